@@ -22,6 +22,7 @@
 
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 
 #include "crp_gpu.h"
 #include "engine_internal.h"
@@ -40,14 +41,8 @@ constexpr double kC = 2.99792458e8;
 struct v3 { double x, y, z; };
 __device__ __forceinline__ v3 mk(double x, double y, double z) { return {x, y, z}; }
 __device__ __forceinline__ v3 add(v3 a, v3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ v3 sub(v3 a, v3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
 __device__ __forceinline__ v3 muls(v3 a, double f) { return {a.x * f, a.y * f, a.z * f}; }
-__device__ __forceinline__ v3 divs(v3 a, double f) { return {a.x / f, a.y / f, a.z / f}; }
 __device__ __forceinline__ double dot(v3 a, v3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ v3 cross(v3 a, v3 v) {
-    return {a.y * v.z - v.y * a.z, a.z * v.x - v.z * a.x, a.x * v.y - v.x * a.y};
-}
-__device__ __forceinline__ double norm(v3 a) { return sqrt(a.x * a.x + a.y * a.y + a.z * a.z); }
 
 struct AdjGrid {
     const float *g;
@@ -55,68 +50,199 @@ struct AdjGrid {
     bool pow2;  // every dimension a power of two: indices wrap with a mask
     double gox, goy, goz, sx, sy, sz;
     double isx, isy, isz;  // 1 / spacing
+    const float *pairs;    // pair records of the values (load_corners), or null
 };
+
+// The pair records are built for grids of up to 2^28 cells (8 GB of
+// workspace); larger grids are read in place.
+constexpr size_t kPairCells = (size_t)1 << 28;
+
+__global__ void pair_kernel(const float *g, int nz, unsigned cells, float4 *pairs) {
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= cells) return;
+    const unsigned j = i % (unsigned)nz == (unsigned)nz - 1 ? i - (unsigned)(nz - 1) : i + 1;
+    const float *a = g + 3 * (size_t)i, *b = g + 3 * (size_t)j;
+    pairs[2 * (size_t)i] = make_float4(__ldg(a), __ldg(a + 1), __ldg(a + 2), 0.f);
+    pairs[2 * (size_t)i + 1] = make_float4(__ldg(b), __ldg(b + 1), __ldg(b + 2), 0.f);
+}
+
+// one 32-byte record in one aligned 256-bit load
+__device__ __forceinline__ void load_pair(const float *p, float a[3], float b[3]) {
+    float pad0, pad1;
+    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(pad0), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(pad1)
+                 : "l"(p));
+}
 
 // periodic index: i mod n in [0, n) (a mask for power-of-two n, the same value)
 __device__ __forceinline__ int wrap_index(int i, int n, bool pow2) {
     return pow2 ? (i & (n - 1)) : ((i % n) + n) % n;
 }
 
-// corner indices, weights and weight gradients of the cell around x
-__device__ __forceinline__ void cell(const AdjGrid &G, v3 x, size_t idx[8], double w[8], double dw[8][3]) {
-    const double r[3] = {(x.x - G.gox) * G.isx, (x.y - G.goy) * G.isy, (x.z - G.goz) * G.isz};
+// A candidate's position on the grid: the lower corner's index and the
+// linear fraction on each axis.
+struct CellPos {
+    int lo[3];
+    double f[3];
+};
+
+// floor(r) of |r| < 2^31 as integer and double without the conversion unit:
+// adding 1.5 * 2^52 towards minus infinity leaves floor(r) in the low mantissa
+// bits.  (The conversions and roundings of FP64 run at a quarter of the FP64
+// rate on sm_100, and the corner loads need 24 of them per step already.)
+__device__ __forceinline__ CellPos locate(const AdjGrid &G, v3 x) {
+    const double magic = 6755399441055744.0;
+    const double r[3] = {__dmul_rn(x.x - G.gox, G.isx), __dmul_rn(x.y - G.goy, G.isy), __dmul_rn(x.z - G.goz, G.isz)};
     const int n[3] = {G.nx, G.ny, G.nz};
-    const double is[3] = {G.isx, G.isy, G.isz};
-    int lo[3], hi[3];
-    double f0[3], f1[3];
+    CellPos c;
+    int i[3];
+    const int big = max(max(__double2hiint(r[0]) & 0x7fffffff, __double2hiint(r[1]) & 0x7fffffff),
+                        __double2hiint(r[2]) & 0x7fffffff);
+    if (big < 0x41e00000) {  // every |r| < 2^31
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
-        double fl = floor(r[a]);
-        lo[a] = wrap_index((int)fl, n[a], G.pow2);
-        hi[a] = G.pow2 ? (lo[a] + 1) & (n[a] - 1) : (lo[a] + 1) % n[a];
-        f0[a] = r[a] - fl;
-        f1[a] = 1 - f0[a];
-    }
-    const int sel[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 0, 1}, {0, 1, 1}, {1, 1, 0}, {1, 1, 1}};
+        for (int a = 0; a < 3; a++) {
+            const double t = __dadd_rd(r[a], magic);
+            i[a] = __double2loint(t);
+            c.f[a] = r[a] - (t - magic);
+        }
+    } else {
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const int ix = sel[k][0] ? hi[0] : lo[0], iy = sel[k][1] ? hi[1] : lo[1], iz = sel[k][2] ? hi[2] : lo[2];
-        idx[k] = ((size_t)ix * G.ny + (size_t)iy) * G.nz + (size_t)iz;
-        const double wx = sel[k][0] ? f0[0] : f1[0], wy = sel[k][1] ? f0[1] : f1[1], wz = sel[k][2] ? f0[2] : f1[2];
-        const double sx = sel[k][0] ? is[0] : -is[0], sy = sel[k][1] ? is[1] : -is[1],
-                     sz = sel[k][2] ? is[2] : -is[2];
-        w[k] = wx * wy * wz;
-        dw[k][0] = sx * wy * wz;
-        dw[k][1] = wx * sy * wz;
-        dw[k][2] = wx * wy * sz;
+        for (int a = 0; a < 3; a++) {
+            const double fl = floor(r[a]);
+            i[a] = (int)fl;
+            c.f[a] = r[a] - fl;
+        }
     }
+#pragma unroll
+    for (int a = 0; a < 3; a++) c.lo[a] = wrap_index(i[a], n[a], G.pow2);
+    return c;
 }
 
-__device__ __forceinline__ v3 field(const AdjGrid &G, const size_t idx[8], const double w[8]) {
+// corner q of the Grid.h:571 order: which of lower / upper on each axis
+__device__ __forceinline__ constexpr int bit(int q, int a) {
+    constexpr int t[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 0, 1}, {0, 1, 1}, {1, 1, 0}, {1, 1, 1}};
+    return t[q][a];
+}
+
+// linear indices of the 8 corners, 32-bit with the pair records (at most
+// kPairCells cells)
+template <class Index>
+__device__ __forceinline__ void corner_indices(const AdjGrid &G, const int lo[3], Index idx[8]) {
+    const Index sx = (Index)G.ny * (Index)G.nz, sy = (Index)G.nz;
+    const Index x0 = (Index)lo[0] * sx, x1 = lo[0] + 1 == G.nx ? 0 : x0 + sx;
+    const Index y0 = (Index)lo[1] * sy, y1 = lo[1] + 1 == G.ny ? 0 : y0 + sy;
+    const Index z0 = (Index)lo[2], z1 = lo[2] + 1 == G.nz ? 0 : z0 + 1;
+#pragma unroll
+    for (int q = 0; q < 8; q++) idx[q] = (bit(q, 0) ? x1 : x0) + (bit(q, 1) ? y1 : y0) + (bit(q, 2) ? z1 : z0);
+}
+
+// The 8 corner values of the cell a candidate is in, held in registers: at
+// 1 kpc per step through 10 kpc cells a candidate leaves its cell on every
+// seventh step or so, and without the cache each step's 24 loads of every lane
+// bound the forward kernel (L1 wavefronts; lg_throttle 4.9 and long_scoreboard
+// 8.1 cycles per issued instruction, 7.0 ms of 10^5 candidates x 2000 steps).
+struct Corners {
+    int lo[3];
+    float v[8][3];
+};
+
+// PAIRS: the grid's copy in pair records, 32 bytes per cell holding the
+// cell's value and its upper z neighbour's, so that a cell's corners are four
+// aligned 256-bit loads instead of 24 scalar ones.
+template <bool PAIRS>
+__device__ __forceinline__ void load_corners(const AdjGrid &G, const CellPos &c, Corners &k) {
+    if (c.lo[0] == k.lo[0] && c.lo[1] == k.lo[1] && c.lo[2] == k.lo[2]) return;
+    if (PAIRS) {
+        unsigned idx[8];
+        corner_indices(G, c.lo, idx);
+        load_pair(G.pairs + 8 * (size_t)idx[0], k.v[0], k.v[3]);
+        load_pair(G.pairs + 8 * (size_t)idx[1], k.v[1], k.v[4]);
+        load_pair(G.pairs + 8 * (size_t)idx[2], k.v[2], k.v[5]);
+        load_pair(G.pairs + 8 * (size_t)idx[6], k.v[6], k.v[7]);
+    } else {
+        size_t idx[8];
+        corner_indices(G, c.lo, idx);
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const float *g = G.g + 3 * idx[q];
+            k.v[q][0] = __ldg(g); k.v[q][1] = __ldg(g + 1); k.v[q][2] = __ldg(g + 2);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) k.lo[a] = c.lo[a];
+}
+
+__device__ __forceinline__ void weights(const CellPos &c, double w[8]) {
+    const double x0 = c.f[0], y0 = c.f[1], z0 = c.f[2], x1 = 1 - x0, y1 = 1 - y0, z1 = 1 - z0;
+    const double a = x1 * y1, b = x0 * y1, d = x1 * y0, e = x0 * y0;
+    w[0] = a * z1; w[1] = b * z1; w[2] = d * z1; w[3] = a * z0;
+    w[4] = b * z0; w[5] = d * z0; w[6] = e * z1; w[7] = e * z0;
+}
+
+__device__ __forceinline__ v3 interpolate(const Corners &k, const double w[8]) {
     v3 B = mk(0, 0, 0);
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const float *c = G.g + 3 * idx[k];
-        B.x += w[k] * (double)__ldg(c);
-        B.y += w[k] * (double)__ldg(c + 1);
-        B.z += w[k] * (double)__ldg(c + 2);
+    for (int q = 0; q < 8; q++) {
+        B.x = fma(w[q], (double)k.v[q][0], B.x);
+        B.y = fma(w[q], (double)k.v[q][1], B.y);
+        B.z = fma(w[q], (double)k.v[q][2], B.z);
     }
     return B;
 }
 
-__device__ __forceinline__ void step(const AdjGrid &G, v3 &x, v3 &u, double hh, double kappa) {
-    v3 x1 = add(x, muls(u, hh));
-    size_t idx[8];
-    double w[8], dw[8][3];
-    cell(G, x1, idx, w, dw);
-    v3 B = field(G, idx, w);
-    v3 t = muls(B, kappa);
-    double D = 1 + dot(t, t);
-    v3 s = muls(t, 2 * (1 / D));
-    v3 v = add(u, cross(u, t));
-    v3 u2 = add(u, cross(v, s));
-    x = add(x1, muls(u2, hh));
-    u = muls(u2, 1 / norm(u2));
+// 1 / D for D = 1 + |t|^2 >= 1 by Newton's iteration from the single-precision
+// reciprocal (relative error 2^-23 -> 2^-46 -> below 2^-52); D beyond the
+// single-precision range (|t| > 10^19, no physical step) divides.
+__device__ __forceinline__ double reciprocal(double D) {
+    if (!(D < 1e38)) return 1 / D;
+    double y = (double)__frcp_rn((float)D);
+    y = fma(y, fma(-D, y, 1.0), y);
+    return fma(y, fma(-D, y, 1.0), y);
+}
+
+// 1 / |u| from n2 = |u|^2.  The Boris rotation preserves |u|, so after the
+// first step n2 is 1 within rounding and one Newton step of 1/sqrt from 1 is
+// exact to rounding (error 3/8 (n2 - 1)^2).
+__device__ __forceinline__ double inverse_norm(double n2) {
+    if (fabs(n2 - 1) > 1e-9) return 1 / sqrt(n2);
+    return fma(-0.5, n2, 1.5);
+}
+
+// a x v and its sum with c, multiply-adds written out: the forward pass and
+// the reverse pass's recomputation have to agree bit for bit.
+__device__ __forceinline__ v3 cross_add(v3 c, v3 a, v3 v) {
+    return mk(fma(-v.y, a.z, fma(a.y, v.z, c.x)), fma(-v.z, a.x, fma(a.z, v.x, c.y)),
+              fma(-v.x, a.y, fma(a.x, v.y, c.z)));
+}
+__device__ __forceinline__ double dotf(v3 a, v3 b) { return fma(a.x, b.x, fma(a.y, b.y, a.z * b.z)); }
+__device__ __forceinline__ v3 axpy(v3 a, double f, v3 c) { return mk(fma(a.x, f, c.x), fma(a.y, f, c.y), fma(a.z, f, c.z)); }
+
+// The Boris rotation of u0 in the field B: u2 = u0 + v x s.
+struct Rotation {
+    v3 t, s, v, u2;
+    double iD;
+};
+
+__device__ __forceinline__ Rotation rotate(v3 u0, v3 B, double kappa) {
+    Rotation r;
+    r.t = muls(B, kappa);
+    r.iD = reciprocal(fma(r.t.x, r.t.x, fma(r.t.y, r.t.y, fma(r.t.z, r.t.z, 1.0))));
+    r.s = muls(r.t, 2 * r.iD);
+    r.v = cross_add(u0, u0, r.t);
+    r.u2 = cross_add(u0, r.v, r.s);
+    return r;
+}
+
+template <bool PAIRS>
+__device__ __forceinline__ void step(const AdjGrid &G, Corners &k, v3 &x, v3 &u, double hh, double kappa) {
+    const v3 x1 = axpy(u, hh, x);
+    const CellPos c = locate(G, x1);
+    load_corners<PAIRS>(G, c, k);
+    double w[8];
+    weights(c, w);
+    const Rotation r = rotate(u, interpolate(k, w), kappa);
+    x = axpy(r.u2, hh, x1);
+    u = muls(r.u2, inverse_norm(dotf(r.u2, r.u2)));
 }
 
 struct IO {
@@ -138,79 +264,81 @@ __global__ void kappa_max_kernel(IO io, double h, unsigned long long *kmax) {
     if ((threadIdx.x & 31) == 0) atomicMax(kmax, b);
 }
 
-// forward pass; with ckpt != null the state before every K-th step is stored
-__global__ void __launch_bounds__(128) forward_kernel(AdjGrid G, IO io, double h, int n_steps, int K,
-                                                      double *ckpt) {
+// forward pass; with ckpt != null the state before every K-th step is stored.
+// Blocks of 64: 10^5 candidates are 1563 blocks, which fill the 148 SMs more
+// evenly than 782 blocks of 128.
+constexpr int kForwardBlock = 64, kReverseBlock = 64;
+
+template <bool PAIRS>
+__global__ void __launch_bounds__(kForwardBlock, 10) forward_kernel(AdjGrid G, IO io, double h, int n_steps, int K,
+                                                                    double *ckpt) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= io.n) return;
     const double kappa = io.charge[i] * h * kC / (2 * io.energy[i]);
     const double hh = h / 2;
     v3 x = mk(io.x[i], io.y[i], io.z[i]), u = mk(io.dx[i], io.dy[i], io.dz[i]);
     const uint64_t n = io.n;
-    for (int k = 0; k < n_steps; k++) {
-        if (ckpt && k % K == 0) {
-            double *c = ckpt + (size_t)(k / K) * 6 * n;
+    Corners corners;
+    corners.lo[0] = -1;
+    const int every = ckpt ? K : n_steps;
+    for (int k0 = 0; k0 < n_steps; k0 += every) {
+        if (ckpt) {
+            double *c = ckpt + (size_t)(k0 / K) * 6 * n;
             c[i] = x.x; c[n + i] = x.y; c[2 * n + i] = x.z;
             c[3 * n + i] = u.x; c[4 * n + i] = u.y; c[5 * n + i] = u.z;
         }
-        step(G, x, u, hh, kappa);
+        const int m = n_steps - k0 < every ? n_steps - k0 : every;
+        for (int k = 0; k < m; k++) step<PAIRS>(G, corners, x, u, hh, kappa);
     }
     io.loss[i] = 1 - dot(u, mk(io.tx[i], io.ty[i], io.tz[i]));
     if (io.ux) { io.ux[i] = u.x; io.uy[i] = u.y; io.uz[i] = u.z; }
 }
 
-// Cell of the periodic grid around x: per-axis lower / upper indices and the
-// linear fractions (corner weights and their gradients are formed from these
-// on the fly, which keeps the reverse kernel's registers in budget).
-struct CellW {
-    int lo[3], hi[3];
-    double f0[3], f1[3];
-};
-
-__device__ __forceinline__ CellW cellw(const AdjGrid &G, v3 x) {
-    CellW c;
-    const double r[3] = {(x.x - G.gox) * G.isx, (x.y - G.goy) * G.isy, (x.z - G.goz) * G.isz};
-    const int n[3] = {G.nx, G.ny, G.nz};
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const double fl = floor(r[a]);
-        c.lo[a] = wrap_index((int)fl, n[a], G.pow2);
-        c.hi[a] = G.pow2 ? (c.lo[a] + 1) & (n[a] - 1) : (c.lo[a] + 1) % n[a];
-        c.f0[a] = r[a] - fl;
-        c.f1[a] = 1 - c.f0[a];
-    }
-    return c;
-}
-
-// corner q of the Grid.h:571 order: which of lo / hi on each axis
-__device__ __forceinline__ int bit(int q, int a) {
-    const int t[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 0, 1}, {0, 1, 1}, {1, 1, 0}, {1, 1, 1}};
-    return t[q][a];
-}
-
-__device__ __forceinline__ size_t corner_index(const AdjGrid &G, const int lo[3], const int hi[3], int q) {
-    const int ix = bit(q, 0) ? hi[0] : lo[0], iy = bit(q, 1) ? hi[1] : lo[1], iz = bit(q, 2) ? hi[2] : lo[2];
-    return ((size_t)ix * G.ny + (size_t)iy) * G.nz + (size_t)iz;
-}
-
-// add one cell's summed contributions to the fixed-point accumulator
-__device__ __forceinline__ void flush(const AdjGrid &G, unsigned long long *acc, const int lo[3],
-                                      const int hi[3], double g[8][3], double scale) {
+// Add one cell's summed contributions to the fixed-point accumulator: g times
+// scale rounded to an integer.  `most` bounds every |g|: where the integers
+// stay below 2^50 the rounding is one multiply-add onto 1.5 * 2^52 and the
+// integer its low mantissa bits (24 FP64-to-integer conversions per flush
+// occupied the conversion unit longer than the multiply-adds do).
+template <bool PAIRS>
+__device__ __forceinline__ void flush(const AdjGrid &G, unsigned long long *acc, const int lo[3], double g[8][3],
+                                      double scale, double &most) {
     if (lo[0] >= 0) {
+        using Index = typename std::conditional<PAIRS, unsigned, size_t>::type;
+        Index idx[8];
+        corner_indices(G, lo, idx);
+        if (most * scale < 1125899906842624.0) {
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-            unsigned long long *a = acc + 3 * corner_index(G, lo, hi, q);
-            atomicAdd(a, (unsigned long long)__double2ll_rn(g[q][0] * scale));
-            atomicAdd(a + 1, (unsigned long long)__double2ll_rn(g[q][1] * scale));
-            atomicAdd(a + 2, (unsigned long long)__double2ll_rn(g[q][2] * scale));
+            for (int q = 0; q < 8; q++)
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    const double t = fma(g[q][a], scale, 6755399441055744.0);
+                    atomicAdd(acc + (3 * idx[q] + a), (unsigned long long)__double_as_longlong(t) - 0x4338000000000000ull);
+                }
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+#pragma unroll
+                for (int a = 0; a < 3; a++)
+                    atomicAdd(acc + (3 * idx[q] + a), (unsigned long long)__double2ll_rn(g[q][a] * scale));
         }
     }
 #pragma unroll
     for (int q = 0; q < 8; q++) g[q][0] = g[q][1] = g[q][2] = 0;
+    most = 0;
 }
 
-__global__ void __launch_bounds__(128, 2) reverse_kernel(AdjGrid G, IO io, double h, int n_steps, int K,
-                                                      const double *ckpt,
+// Bound by the issue and latency of some 620 instructions per step (250 of
+// them FP64) at the warps its registers allow: 6 blocks of 64 (168 registers,
+// of which 72 hold the cell's corners and gradient sums).  Measured over 10^5
+// candidates x 2000 steps, 128^3 grid, checkpoints every 100, forward and
+// reverse kernels with their Python wrapper: 27.3 ms before the corner cache,
+// pair records, Newton reciprocals and FP64-to-integer rounding by addition;
+// 19.2 ms now (forward pass 8.5 -> 3.5 ms); 25.2 ms at 8 blocks (128
+// registers, 656 B of spills), 19.5 ms at 5.
+constexpr int kReverseMinBlocks = 6;
+template <bool PAIRS>
+__global__ void __launch_bounds__(kReverseBlock, kReverseMinBlocks) reverse_kernel(AdjGrid G, IO io, double h,
+                                                      int n_steps, int K, const double *ckpt,
                                                       unsigned long long *acc,
                                                       const unsigned long long *kmax_bits) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -220,95 +348,87 @@ __global__ void __launch_bounds__(128, 2) reverse_kernel(AdjGrid G, IO io, doubl
     const double hh = h / 2;
     const double kmax = __longlong_as_double((long long)*kmax_bits);
     const double scale = (acc && kmax > 0) ? ldexp(1.0 / kmax, 36) : 0.0;
-    const double is[3] = {G.isx, G.isy, G.isz};
     v3 xs[kMaxK], us[kMaxK];
     v3 xb = mk(0, 0, 0), ub = mk(-io.tx[i], -io.ty[i], -io.tz[i]);
     double kb = 0;
-    // the cell the candidate is in: its corner values, and its grid-gradient
-    // contributions summed in registers and flushed with atomics when the
-    // candidate leaves the cell
-    int clo[3] = {-1, -1, -1}, chi[3] = {-1, -1, -1};
-    float gc[8][3];
-    double gacc[8][3];
+    // the cell the candidate is in: its corner values (shared by the
+    // recomputation and the reverse steps), and the grid-gradient
+    // contributions of the cell glo, summed in registers and flushed with
+    // atomics when the reverse steps leave it
+    Corners corners;
+    corners.lo[0] = -1;
+    int glo[3] = {-1, -1, -1};
+    double gacc[8][3], most = 0;
 #pragma unroll
     for (int q = 0; q < 8; q++) gacc[q][0] = gacc[q][1] = gacc[q][2] = 0;
     const int nseg = (n_steps + K - 1) / K;
     for (int j = nseg - 1; j >= 0; j--) {
         const double *c = ckpt + (size_t)j * 6 * n;
-        const int k0 = j * K, k1 = (k0 + K < n_steps) ? k0 + K : n_steps;
+        const int m = (j * K + K < n_steps) ? K : n_steps - j * K;
         v3 x = mk(c[i], c[n + i], c[2 * n + i]), u = mk(c[3 * n + i], c[4 * n + i], c[5 * n + i]);
-        // the states before each step of the segment (the segment's own end
-        // state is not needed: checkpoint_every = 1 recomputes nothing)
-        for (int k = k0; k < k1; k++) {
-            xs[k - k0] = x; us[k - k0] = u;
-            if (k + 1 < k1) step(G, x, u, hh, kappa);
+        // the states before each step of the segment (the last one stays in x
+        // and u: checkpoint_every = 1 recomputes and stores nothing)
+        for (int k = 0; k + 1 < m; k++) {
+            xs[k] = x; us[k] = u;
+            step<PAIRS>(G, corners, x, u, hh, kappa);
         }
-        for (int k = k1 - 1; k >= k0; k--) {
-            const v3 u0 = us[k - k0];
-            const v3 x1 = add(xs[k - k0], muls(u0, hh));
-            const CellW cw = cellw(G, x1);
-            // a new cell: flush the previous cell's gradient, load this one's corners
-            // (a candidate stays in one cell for several steps)
-            if (cw.lo[0] != clo[0] || cw.lo[1] != clo[1] || cw.lo[2] != clo[2] || cw.hi[0] != chi[0] ||
-                cw.hi[1] != chi[1] || cw.hi[2] != chi[2]) {
-                if (acc) flush(G, acc, clo, chi, gacc, scale);
+        for (int k = m - 1; k >= 0; k--) {
+            const v3 u0 = u;
+            const CellPos cp = locate(G, axpy(u0, hh, x));
+            // the state before the previous step, asked for a step ahead
+            if (k > 0) { x = xs[k - 1]; u = us[k - 1]; }
+            if (acc && (cp.lo[0] != glo[0] || cp.lo[1] != glo[1] || cp.lo[2] != glo[2])) {
+                flush<PAIRS>(G, acc, glo, gacc, scale, most);
 #pragma unroll
-                for (int a = 0; a < 3; a++) { clo[a] = cw.lo[a]; chi[a] = cw.hi[a]; }
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    const float *cg = G.g + 3 * corner_index(G, cw.lo, cw.hi, q);
-                    gc[q][0] = __ldg(cg); gc[q][1] = __ldg(cg + 1); gc[q][2] = __ldg(cg + 2);
-                }
+                for (int a = 0; a < 3; a++) glo[a] = cp.lo[a];
             }
-            v3 B = mk(0, 0, 0);
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const double wq = (bit(q, 0) ? cw.f0[0] : cw.f1[0]) * (bit(q, 1) ? cw.f0[1] : cw.f1[1]) *
-                                  (bit(q, 2) ? cw.f0[2] : cw.f1[2]);
-                B.x += wq * (double)gc[q][0];
-                B.y += wq * (double)gc[q][1];
-                B.z += wq * (double)gc[q][2];
-            }
-            const v3 t = muls(B, kappa);
-            const double D = 1 + dot(t, t);
-            const double iD = 1 / D;
-            const v3 s = muls(t, 2 * iD);
-            const v3 v = add(u0, cross(u0, t));
-            const v3 u2 = add(u0, cross(v, s));
-            const double inn = 1 / norm(u2);
-            const v3 un = muls(u2, inn);
+            load_corners<PAIRS>(G, cp, corners);
+            double w[8];
+            weights(cp, w);
+            const v3 B = interpolate(corners, w);
+            const Rotation r = rotate(u0, B, kappa);
+            const double inn = inverse_norm(dotf(r.u2, r.u2));
+            const v3 un = muls(r.u2, inn);
             // reverse of: normalisation, second half drift, Boris rotation
-            v3 u2b = muls(sub(ub, muls(un, dot(un, ub))), inn);
-            u2b = add(u2b, muls(xb, hh));
-            const v3 vb = cross(s, u2b);
-            const v3 sb = cross(u2b, v);
-            const v3 ubar = add(u2b, add(vb, cross(t, vb)));
-            v3 tb = cross(vb, u0);
-            tb = add(tb, sub(muls(sb, 2 * iD), muls(t, 4 * dot(t, sb) * (iD * iD))));
+            v3 u2b = muls(axpy(un, -dotf(un, ub), ub), inn);
+            u2b = axpy(xb, hh, u2b);
+            const v3 vb = cross_add(mk(0, 0, 0), r.s, u2b);
+            const v3 sb = cross_add(mk(0, 0, 0), u2b, r.v);
+            const v3 ubar = cross_add(add(u2b, vb), r.t, vb);
+            v3 tb = axpy(sb, 2 * r.iD, cross_add(mk(0, 0, 0), vb, u0));
+            tb = axpy(r.t, -4 * dotf(r.t, sb) * (r.iD * r.iD), tb);
             const v3 Bb = muls(tb, kappa);
-            kb += dot(tb, B);
-            // reverse of the interpolation: position Jacobian and grid values
-            v3 x1b = xb;
+            most += fabs(Bb.x) + fabs(Bb.y) + fabs(Bb.z);
+            kb = fma(tb.x, B.x, fma(tb.y, B.y, fma(tb.z, B.z, kb)));
+            // reverse of the interpolation.  Grid values: weight times Bb.
+            // Position: the gradient of the trilinear form of g_q = Bb . c_q by
+            // differences and lerps, z first, corners g[x][y][z].
+            double g[2][2][2];
 #pragma unroll
             for (int q = 0; q < 8; q++) {
-                const double wx = bit(q, 0) ? cw.f0[0] : cw.f1[0], wy = bit(q, 1) ? cw.f0[1] : cw.f1[1],
-                             wz = bit(q, 2) ? cw.f0[2] : cw.f1[2];
-                const double sx = bit(q, 0) ? is[0] : -is[0], sy = bit(q, 1) ? is[1] : -is[1],
-                             sz = bit(q, 2) ? is[2] : -is[2];
-                const double gdot = Bb.x * (double)gc[q][0] + Bb.y * (double)gc[q][1] + Bb.z * (double)gc[q][2];
-                x1b.x += gdot * (sx * wy * wz);
-                x1b.y += gdot * (wx * sy * wz);
-                x1b.z += gdot * (wx * wy * sz);
-                const double wq = wx * wy * wz;
-                gacc[q][0] += wq * Bb.x;
-                gacc[q][1] += wq * Bb.y;
-                gacc[q][2] += wq * Bb.z;
+                g[bit(q, 0)][bit(q, 1)][bit(q, 2)] =
+                    fma(Bb.x, (double)corners.v[q][0],
+                        fma(Bb.y, (double)corners.v[q][1], Bb.z * (double)corners.v[q][2]));
+                gacc[q][0] = fma(w[q], Bb.x, gacc[q][0]);
+                gacc[q][1] = fma(w[q], Bb.y, gacc[q][1]);
+                gacc[q][2] = fma(w[q], Bb.z, gacc[q][2]);
             }
-            xb = x1b;
-            ub = add(ubar, muls(x1b, hh));
+            double a[2], dy[2], dz[2];
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+                const double z0 = g[p][0][1] - g[p][0][0], z1 = g[p][1][1] - g[p][1][0];
+                const double h0 = fma(cp.f[2], z0, g[p][0][0]), h1 = fma(cp.f[2], z1, g[p][1][0]);
+                dz[p] = fma(cp.f[1], z1 - z0, z0);
+                dy[p] = h1 - h0;
+                a[p] = fma(cp.f[1], dy[p], h0);
+            }
+            xb.x = fma(a[1] - a[0], G.isx, xb.x);
+            xb.y = fma(fma(cp.f[0], dy[1] - dy[0], dy[0]), G.isy, xb.y);
+            xb.z = fma(fma(cp.f[0], dz[1] - dz[0], dz[0]), G.isz, xb.z);
+            ub = axpy(xb, hh, ubar);
         }
     }
-    if (acc) flush(G, acc, clo, chi, gacc, scale);
+    if (acc) flush<PAIRS>(G, acc, glo, gacc, scale, most);
     io.gdx[i] = ub.x; io.gdy[i] = ub.y; io.gdz[i] = ub.z;
     io.ge[i] = kb * (-kappa / io.energy[i]);
 }
@@ -359,6 +479,7 @@ AdjGrid make_grid(const crp_adjoint_desc *d) {
     G.goz = d->origin[2] + d->spacing[2] / 2;
     G.sx = d->spacing[0]; G.sy = d->spacing[1]; G.sz = d->spacing[2];
     G.isx = 1.0 / G.sx; G.isy = 1.0 / G.sy; G.isz = 1.0 / G.sz;
+    G.pairs = nullptr;
     return G;
 }
 
@@ -383,8 +504,9 @@ crp_status crp_bp_adjoint_workspace(const crp_adjoint_desc *d, uint64_t n, size_
     if (d->checkpoint_every < 1 || d->checkpoint_every > kMaxK)
         return fail(CRP_ERR_CAPACITY, "checkpoint_every must be 1..128");
     const size_t nck = (size_t)((d->n_steps + d->checkpoint_every - 1) / d->checkpoint_every);
-    *bytes = align256(256) + align256(nck * 6 * n * sizeof(double)) +
-             align256((size_t)d->nx * d->ny * d->nz * 3 * sizeof(unsigned long long));
+    const size_t cells = (size_t)d->nx * d->ny * d->nz;
+    *bytes = align256(256) + align256(nck * 6 * n * sizeof(double)) + align256(cells * 3 * sizeof(unsigned long long)) +
+             (cells <= kPairCells ? align256(cells * 8 * sizeof(float)) : 0);
     return CRP_OK;
 }
 
@@ -392,7 +514,7 @@ crp_status crp_bp_forward_loss(const crp_adjoint_desc *d, const crp_adjoint_io *
     crp_status st = check_desc(d, a);
     if (st) return st;
     if (a->n == 0) return CRP_OK;
-    forward_kernel<<<(unsigned)((a->n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(
+    forward_kernel<false><<<(unsigned)((a->n + kForwardBlock - 1) / kForwardBlock), kForwardBlock, 0, (cudaStream_t)stream>>>(
         make_grid(d), make_io(a), d->step, d->n_steps, d->checkpoint_every, nullptr);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CRP_OK : cuda_fail(e, "adjoint forward kernel launch");
@@ -417,23 +539,39 @@ static crp_status adjoint_impl(const crp_adjoint_desc *d, const crp_adjoint_io *
     double *ckpt = reinterpret_cast<double *>(w + align256(256));
     const size_t cells3 = (size_t)d->nx * d->ny * d->nz * 3;
     unsigned long long *acc = reinterpret_cast<unsigned long long *>(w + align256(256) + align256(nck * 6 * a->n * sizeof(double)));
-    const AdjGrid G = make_grid(d);
+    AdjGrid G = make_grid(d);
+    const size_t cells = cells3 / 3;
+    if (cells <= kPairCells)
+        G.pairs = reinterpret_cast<const float *>(reinterpret_cast<char *>(acc) + align256(cells3 * sizeof(unsigned long long)));
     const IO io = make_io(a);
-    const unsigned blocks = (unsigned)((a->n + 127) / 128);
+    auto blocks = [&](unsigned threads) { return (unsigned)((a->n + threads - 1) / threads); };
     cudaError_t e = cudaSuccess;
     if (do_forward) {
         e = cudaMemsetAsync(kmax, 0, 8, s);
         if (e != cudaSuccess) return cuda_fail(e, "clearing the adjoint workspace");
-        kappa_max_kernel<<<blocks, 128, 0, s>>>(io, d->step, kmax);
-        forward_kernel<<<blocks, 128, 0, s>>>(G, io, d->step, d->n_steps, d->checkpoint_every, ckpt);
+        kappa_max_kernel<<<blocks(128), 128, 0, s>>>(io, d->step, kmax);
+        if (G.pairs) {
+            pair_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(
+                G.g, G.nz, (unsigned)cells, reinterpret_cast<float4 *>(const_cast<float *>(G.pairs)));
+            forward_kernel<true><<<blocks(kForwardBlock), kForwardBlock, 0, s>>>(G, io, d->step, d->n_steps,
+                                                                                 d->checkpoint_every, ckpt);
+        } else {
+            forward_kernel<false><<<blocks(kForwardBlock), kForwardBlock, 0, s>>>(G, io, d->step, d->n_steps,
+                                                                                  d->checkpoint_every, ckpt);
+        }
     }
     if (do_backward) {
         if (a->grad_grid) {
             e = cudaMemsetAsync(acc, 0, cells3 * sizeof(unsigned long long), s);
             if (e != cudaSuccess) return cuda_fail(e, "clearing the adjoint workspace");
         }
-        reverse_kernel<<<blocks, 128, 0, s>>>(G, io, d->step, d->n_steps, d->checkpoint_every, ckpt,
-                                              a->grad_grid ? acc : nullptr, kmax);
+        unsigned long long *grad = a->grad_grid ? acc : nullptr;
+        if (G.pairs)
+            reverse_kernel<true><<<blocks(kReverseBlock), kReverseBlock, 0, s>>>(G, io, d->step, d->n_steps,
+                                                                                 d->checkpoint_every, ckpt, grad, kmax);
+        else
+            reverse_kernel<false><<<blocks(kReverseBlock), kReverseBlock, 0, s>>>(G, io, d->step, d->n_steps,
+                                                                                  d->checkpoint_every, ckpt, grad, kmax);
         if (a->grad_grid)
             finalize_kernel<<<(unsigned)((cells3 + 255) / 256), 256, 0, s>>>(acc, cells3, kmax, a->grad_grid);
     }

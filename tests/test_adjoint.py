@@ -107,3 +107,37 @@ def test_autograd_function_gives_momentum_and_grid_gradients():
     np.testing.assert_allclose(p0.grad.cpu().numpy(), gp_expected, rtol=1e-9, atol=1e-12 * np.abs(gp_expected).max())
     np.testing.assert_allclose(g.grad.cpu().numpy(), gg.astype(np.float32), rtol=1e-6, atol=1e-6 * np.abs(gg).max())
     assert abs(L.item() - _gpu(grid, pos, u0, energy, charge, target, want_grid=False)[0].sum()) < 1e-9
+
+
+@pytest.mark.parametrize("shape,n", [((1, 1, 1), 3), ((5, 7, 3), 65), ((16, 16, 16), 64), ((2, 9, 4), 129)])
+def test_adjoint_at_odd_grids_and_batches(oracle, shape, n):
+    """Cell wrap on grids of any size, partial blocks, positions far outside
+    the grid, and the loss of the pass without pair records (bp_forward_loss)
+    bit for bit."""
+    import torch
+    from crpropa3_b200.adjoint import bp_forward_loss, bp_loss_and_grads
+    rng = np.random.default_rng(84 + n)
+    grid = (rng.standard_normal(shape + (3,)) * 3e-13).astype(np.float32)
+    u0 = stable_unit_vectors(rng, n)
+    energy = np.exp(rng.uniform(np.log(5), np.log(50), n)) * U.EeV
+    charge = np.full(n, -U.eplus)
+    pos = rng.uniform(-500, 500, (n, 3)) * U.kpc
+    target = stable_unit_vectors(rng, n)
+    ref = oracle.bp_adjoint(grid, ORIGIN, SPACING, STEP, 60, pos, u0, energy, charge, target)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    args = (t(grid), ORIGIN, SPACING, STEP, 60, t(pos), t(u0), t(energy), t(charge), t(target))
+    got = bp_loss_and_grads(*args, checkpoint_every=9)
+    for g, r, tol in zip(got, ref, (1e-13, 1e-12, 1e-12, 1e-9)):
+        g = g.cpu().numpy()
+        np.testing.assert_allclose(g, r, rtol=0, atol=tol * max(np.abs(r).max(), 1e-300))
+    np.testing.assert_array_equal(got[0].cpu().numpy(), bp_forward_loss(*args)[0].cpu().numpy())
+
+
+def test_adjoint_of_directions_off_unit_length(oracle):
+    """The first step normalises whatever direction it is given."""
+    grid, pos, u0, energy, charge, target = _problem(n=33, seed=85)
+    u0 = u0 * np.random.default_rng(85).uniform(0.5, 2.0, (33, 1))
+    ref = oracle.bp_adjoint(grid, ORIGIN, SPACING, STEP, NSTEPS, pos, u0, energy, charge, target)
+    got = _gpu(grid, pos, u0, energy, charge, target)
+    for g, r, tol in zip(got, ref, (1e-12, 1e-10, 1e-10, 1e-9)):
+        np.testing.assert_allclose(g, r, rtol=0, atol=tol * np.abs(r).max())
