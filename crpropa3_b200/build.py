@@ -1,6 +1,6 @@
 """Build the engine library crpropa3_b200/lib/libcrp_b200.so for sm_100a.
 
-nvcc cross-compiles without a GPU.  The FP64 stepping translation unit is
+nvcc cross-compiles without a GPU.  The FP64 stepping translation units are
 compiled with -fmad=false so that no multiply-add is contracted (bit parity
 with the reference built without FMA); the other units use the default
 contraction.  Objects go to _build/ at the repository root.
@@ -29,8 +29,11 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + INCLUD
 # source -> extra flags
 SOURCES = {
     "step_fp64.cu": ["-fmad=false"],
+    "step_fp64_bp.cu": ["-fmad=false"],
+    "step_fp64_ck.cu": ["-fmad=false"],
     "step_mixed.cu": [],
     "step_mixed_bp.cu": [],
+    "step_mixed_ck.cu": [],
     "adjoint.cu": [],
     "turbulence.cu": [],
     "crp_engine.cu": [],
@@ -78,7 +81,8 @@ def _compile(nvcc, src, flags, verbose):
         return out
     cmd = [nvcc] + ARCH + COMMON + flags
     if src.endswith(".cu"):
-        cmd += ["-Xptxas", "-v"]
+        # the stepping units hold dozens of large kernels: optimised in parallel
+        cmd += ["-Xptxas", "-v", "--split-compile=4"]
     cmd += ["-c", path, "-o", out]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:

@@ -30,8 +30,38 @@ struct Cand {
     // one cell for several steps, so the gathers are skipped while it does;
     // the values are the grid's own, so results do not change.
     long long cell0, cell7;
+    unsigned tag;  // periodic power-of-two grids: the first corner's index alone
     float corner[8][3];
 };
+
+// floor of the three grid coordinates, as integers (low 32 bits) and as
+// doubles.  FP64 roundings and FP64-to-integer conversions run on the
+// conversion unit at a quarter of the FP64 rate; for |r| < 2^31 adding
+// 1.5 * 2^52 towards minus infinity leaves floor(r) in the low mantissa bits,
+// and subtracting it again gives floor(r) exactly.
+struct CellIndex {
+    int ix, iy, iz;
+    double flx, fly, flz;
+};
+
+__device__ __forceinline__ CellIndex cell_index(double rx, double ry, double rz) {
+    const double magic = 6755399441055744.0;
+    const int big = max(max(__double2hiint(rx) & 0x7fffffff, __double2hiint(ry) & 0x7fffffff),
+                        __double2hiint(rz) & 0x7fffffff);
+    CellIndex c;
+    if (big < 0x41e00000) {
+        const double tx = __dadd_rd(rx, magic), ty = __dadd_rd(ry, magic), tz = __dadd_rd(rz, magic);
+        c.ix = __double2loint(tx); c.iy = __double2loint(ty); c.iz = __double2loint(tz);
+        c.flx = tx - magic; c.fly = ty - magic; c.flz = tz - magic;
+    } else {
+        c.flx = floor(rx); c.fly = floor(ry); c.flz = floor(rz);
+        c.ix = (int)c.flx; c.iy = (int)c.fly; c.iz = (int)c.flz;
+    }
+    return c;
+}
+
+constexpr unsigned kNoCell = 0xffffffffu;  // periodic grids have fewer than 2^31 cells
+
 
 __device__ __forceinline__ void load_cand(const DevState &s, uint64_t i, Cand &c) {
     c.x = s.x[i]; c.y = s.y[i]; c.z = s.z[i];
@@ -47,6 +77,7 @@ __device__ __forceinline__ void load_cand(const DevState &s, uint64_t i, Cand &c
     c.active = s.active[i] != 0;
     c.cell0 = -1;
     c.cell7 = -1;
+    c.tag = kNoCell;
 }
 
 __device__ __forceinline__ void store_cand(const DevState &s, const Cand &c) {
@@ -58,6 +89,34 @@ __device__ __forceinline__ void store_cand(const DevState &s, const Cand &c) {
     if (s.steps) s.steps[i] = c.steps;
     s.flags[i] = c.flags;
     s.active[i] = c.active ? 1 : 0;
+}
+
+// One 32-byte pair record (DevGrid::pairs): one 256-bit load, or two 128-bit
+// ones in functions that are not inlined (ptxas 12.9 crashes on a 256-bit load
+// in a function that several kernels call).
+template <bool WIDE>
+__device__ __forceinline__ void load_pair(const float *p, float a[3], float b[3]) {
+    if (!WIDE) {
+        const float4 u = __ldg(reinterpret_cast<const float4 *>(p)), v = __ldg(reinterpret_cast<const float4 *>(p) + 1);
+        a[0] = u.x; a[1] = u.y; a[2] = u.z;
+        b[0] = v.x; b[1] = v.y; b[2] = v.z;
+        return;
+    }
+    float pad0, pad1;
+    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(pad0), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(pad1)
+                 : "l"(p));
+}
+
+// The 8 corners (order of Grid.h:571) of the cell with lower z index iz0 and
+// the four (x, y) columns at b00 .. b11, from the pair records.
+template <bool WIDE, class Index>
+__device__ __forceinline__ void load_corner_pairs(const float *pairs, Index b00, Index b10, Index b01, Index b11,
+                                                  int iz0, float c[8][3]) {
+    load_pair<WIDE>(pairs + 8 * (size_t)(b00 + iz0), c[0], c[3]);
+    load_pair<WIDE>(pairs + 8 * (size_t)(b10 + iz0), c[1], c[4]);
+    load_pair<WIDE>(pairs + 8 * (size_t)(b01 + iz0), c[2], c[5]);
+    load_pair<WIDE>(pairs + 8 * (size_t)(b11 + iz0), c[6], c[7]);
 }
 
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11).
@@ -154,6 +213,34 @@ __device__ __forceinline__ double dmin_std(double a, double b) { return (b < a) 
 __device__ __forceinline__ double dmax_std(double a, double b) { return (a < b) ? b : a; }  // std::max
 // Candidate::limitNextStep (Candidate.cpp:102)
 __device__ __forceinline__ void limit_next(Cand &c, double step) { c.next = (step < c.next) ? step : c.next; }
+
+// The step controller of PropagationCK::process (PropagationCK.cpp:108) and
+// PropagationBP::process (PropagationBP.cpp:96) for an error ratio r: newStep
+// = step * 0.95 * r^-0.2 within [0.1, 5] times the step and the module's
+// limits.  Returns true when the try is rejected (step stays, newStep is the
+// next try's).  The power (250 FP64 instructions and more) is only evaluated
+// where its value survives the limits: below r = 2.4e-4 the factor
+// 0.95 r^-0.2 is above 5, and a single-precision estimate (relative error
+// below 1e-5) that passes a module limit by 1e-3 decides that limit.
+template <class Pow>
+__device__ __forceinline__ bool step_control(const DevModule &m, double r, double step, double &newStep, Pow power) {
+    const bool over = r > 1;
+    newStep = step;
+    if (over ? step == m.min_step : step == m.max_step) return false;
+    const double least = 0.1 * step, most = 5 * step;
+    const float est = (float)step * 0.95f * exp2f(-0.2f * __log2f((float)r));
+    if (!over && r < 2.4e-4) {
+        newStep = dmin_std(most, m.max_step);
+    } else if (!over && est * 0.999f > (float)m.max_step) {
+        newStep = dmin_std(most, m.max_step);
+    } else if (over && r < 1e37 && est * 1.001f < (float)m.min_step) {
+        newStep = dmax_std(least, m.min_step);
+    } else {
+        const double want = step * 0.95 * power(r, -0.2);
+        newStep = over ? dmax_std(dmax_std(want, least), m.min_step) : dmin_std(dmin_std(want, most), m.max_step);
+    }
+    return over;
+}
 
 // ParticleID.cpp:37 isNucleus (neutron counted) with HepPID::isNucleus
 // (ParticleIDMethods.cc:242): proton, or +/-10LZZZAAAI with A >= Z.
@@ -287,27 +374,76 @@ __device__ __forceinline__ void boundary(const DevModule &m, Cand &c, const DevR
     }
 }
 
-// ModuleList::process (ModuleList.cpp.in:54): every module of the chain, in
-// order, whether or not an earlier module deactivated the candidate; a
-// compiled module sequence for the chain shapes of device_plan.cuh, else the
-// module list walked in order.
-template <class Prop, int CS = CS_GENERIC>
-__device__ __forceinline__ void chain_process(const DevPlan &P, Cand &c, const DevRecords &rec,
-                                              StepCount &sc) {
-    if (CS == CS_PM || CS == CS_PMO) {
-        Prop::process(P, P.modules[0], c, sc);
-        max_trajectory_length(P.modules[1], c, rec, 1);
-        if (CS == CS_PMO) observer(P, P.modules[2], c, rec, 2);
-        return;
-    }
+// The non-propagation modules mi in [from, to) of one chain iteration.
+__device__ __forceinline__ void chain_part(const DevPlan &P, Cand &c, const DevRecords &rec, int from, int to) {
 #pragma unroll 1
-    for (int mi = 0; mi < P.n_modules; mi++) {
+    for (int mi = from; mi < to; mi++) {
         const DevModule &m = P.modules[mi];
-        if (m.kind == CRP_MODULE_PROPAGATION) Prop::process(P, m, c, sc);
-        else if (m.kind == CRP_MODULE_MAX_TRAJECTORY_LENGTH) max_trajectory_length(m, c, rec, mi);
+        if (m.kind == CRP_MODULE_MAX_TRAJECTORY_LENGTH) max_trajectory_length(m, c, rec, mi);
         else if (m.kind == CRP_MODULE_OBSERVER) observer(P, m, c, rec, mi);
-        else boundary(m, c, rec, mi);
+        else if (m.kind == CRP_MODULE_BOUNDARY) boundary(m, c, rec, mi);
     }
+}
+
+// Up to kmax iterations of the chain (ModuleList::process,
+// ModuleList.cpp.in:54: every module in order, whether or not an earlier one
+// deactivated the candidate), with a compiled module sequence for the chain
+// shapes of device_plan.cuh; returns the iterations made.  All lanes of a warp
+// call it together, those without a candidate with c.active false.
+//
+// The loop is over tries of the propagation module's step, not over steps: a
+// lane whose try its step controller rejects tries again in the next pass
+// beside the lanes that start their next step.  With the retries in a loop of
+// their own inside the step, a warp made as many tries in each step as its
+// worst lane (nuclei over the 256^3 grid: 2.1 tries per step on average, 5.7
+// of 32 lanes active).
+template <class Prop, int CS>
+__device__ __forceinline__ int advance(const DevPlan &P, Cand &c, const DevRecords &rec, StepCount &sc, int kmax) {
+    const int pi = CS == CS_GENERIC ? P.prop_index : 0;
+    const DevModule &pm = P.modules[pi];
+    typename Prop::Try t;
+    int k = 0;
+    auto rest = [&]() {  // the chain after the propagation module
+        if (CS == CS_GENERIC) {
+            chain_part(P, c, rec, pi + 1, P.n_modules);
+        } else {
+            max_trajectory_length(P.modules[1], c, rec, 1);
+            if (CS == CS_PMO) observer(P, P.modules[2], c, rec, 2);
+        }
+        // c.steps is kept current only for modules that read it
+        if (Prop::kReadsStepCount) c.steps++;
+        k++;
+    };
+    if (!Prop::kRetries) {
+        while (c.active && k < kmax) {
+            if (CS == CS_GENERIC) chain_part(P, c, rec, 0, pi);
+            if (Prop::begin(P, pm, c, t)) Prop::attempt(P, pm, c, t, sc);
+            rest();
+        }
+    } else {
+        bool open = false;  // a step whose tries were all rejected so far
+        // the vote brings the warp's lanes together before every pass
+        while (__any_sync(0xffffffffu, open || (c.active && k < kmax))) {
+            bool done = false;
+            if (!open && c.active && k < kmax) {
+                if (CS == CS_GENERIC) chain_part(P, c, rec, 0, pi);
+                open = Prop::begin(P, pm, c, t);
+                done = !open;  // a neutral candidate's step needs no try
+            }
+            // one copy of the try for the lanes that begin a step and those that
+            // repeat one: without the barrier the compiler may compile the two
+            // paths apart, and a warp then runs them one after the other (10^5
+            // nuclei 61 ms and 117 ms, adaptive Boris push 2.6 and 4.1 ms)
+            __syncwarp();
+            if (open) {
+                done = Prop::attempt(P, pm, c, t, sc);
+                open = !done;
+            }
+            if (done) rest();
+        }
+    }
+    if (!Prop::kReadsStepCount) c.steps += (uint64_t)k;
+    return k;
 }
 
 __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
@@ -344,43 +480,52 @@ __device__ __forceinline__ void append_active(DevCounters *cnt, uint32_t *list, 
     if (still && list) list[base + __popc(mask & ((1u << lane) - 1u))] = index;
 }
 
+// The candidate slot of this thread: each warp takes `lanes` consecutive
+// slots (32: one per lane).  Small runs take fewer than 32 (lanes_per_warp,
+// engine_internal.h).
+__device__ __forceinline__ uint64_t candidate_slot(int lanes, uint64_t n) {
+    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned lane = threadIdx.x & 31;
+    return lane < (unsigned)lanes ? w * (unsigned)lanes + lane : n;
+}
+
+// Iterations this launch may take: max_steps, and what the per-candidate cap
+// leaves.
+__device__ __forceinline__ int launch_steps(const Cand &c, int max_steps, uint64_t step_cap) {
+    if (!step_cap) return max_steps;
+    const uint64_t left = step_cap > c.steps ? step_cap - c.steps : 0;
+    return left < (uint64_t)max_steps ? (int)left : max_steps;
+}
+
 // One thread per candidate, at most max_steps chain iterations per launch.
-// perm_in (optional) maps thread -> candidate index; the candidates still
+// perm_in (optional) maps slot -> candidate index; the candidates still
 // active afterwards are appended to perm_out (optional).
 template <class Prop, int CS = CS_GENERIC>
-__device__ __forceinline__ void chunk_body(const DevPlan &P, const DevState &s, uint64_t n,
+__device__ __forceinline__ void chunk_body(const DevPlan &P, const DevState &s, uint64_t n, int lanes,
                                            int max_steps, uint64_t step_cap,
                                            DevCounters *cnt, const DevRecords &rec,
                                            const uint32_t *perm_in, uint32_t *perm_out) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t t = candidate_slot(lanes, n);
     StepCount sc;
     unsigned long long steps = 0;
     bool still = false;
     uint64_t i = 0;
+    Cand c;
+    c.active = false;
+    int kmax = 0;
+    bool loaded = false;
     if (t < n) {
         i = perm_in ? perm_in[t] : t;
         if (s.active[i]) {
-            Cand c;
             load_cand(s, i, c);
-            // iterations this launch may take: max_steps, and what the
-            // per-candidate cap leaves; c.steps is kept current inside the
-            // loop only for modules that read it (Prop::kReadsStepCount)
-            int kmax = max_steps;
-            if (step_cap) {
-                const uint64_t left = step_cap > c.steps ? step_cap - c.steps : 0;
-                kmax = left < (uint64_t)kmax ? (int)left : kmax;
-            }
-            int k = 0;
-            while (c.active && k < kmax) {
-                chain_process<Prop, CS>(P, c, rec, sc);
-                if (Prop::kReadsStepCount) c.steps++;
-                k++;
-            }
-            if (!Prop::kReadsStepCount) c.steps += (uint64_t)k;
-            steps = (unsigned long long)k;
-            still = c.active && (step_cap == 0 || c.steps < step_cap);
-            store_cand(s, c);
+            kmax = launch_steps(c, max_steps, step_cap);
+            loaded = true;
         }
+    }
+    steps = (unsigned long long)advance<Prop, CS>(P, c, rec, sc, kmax);
+    if (loaded) {
+        still = c.active && (step_cap == 0 || c.steps < step_cap);
+        store_cand(s, c);
     }
     flush_counters(cnt, steps, sc);
     append_active(cnt, perm_out, still, (uint32_t)i);
@@ -418,6 +563,7 @@ __device__ __forceinline__ void persistent_body(const DevPlan &P, const DevState
     Cand c;
     c.cell0 = -1;
     c.cell7 = -1;
+    c.tag = kNoCell;
     bool has = false, exhausted = false;
     for (;;) {
         const unsigned freemask = __ballot_sync(full, !has);
@@ -442,24 +588,10 @@ __device__ __forceinline__ void persistent_body(const DevPlan &P, const DevState
             if (exhausted) break;
             continue;
         }
-        if (has) {
-            int kmax = burst;
-            if (step_cap) {
-                const uint64_t left = step_cap > c.steps ? step_cap - c.steps : 0;
-                kmax = left < (uint64_t)kmax ? (int)left : kmax;
-            }
-            int k = 0;
-            while (c.active && k < kmax) {
-                chain_process<Prop, CS>(P, c, rec, sc);
-                if (Prop::kReadsStepCount) c.steps++;
-                k++;
-            }
-            if (!Prop::kReadsStepCount) c.steps += (uint64_t)k;
-            steps += (unsigned long long)k;
-            if (!c.active || (step_cap != 0 && c.steps >= step_cap)) {
-                store_cand(s, c);
-                has = false;
-            }
+        steps += (unsigned long long)advance<Prop, CS>(P, c, rec, sc, has ? launch_steps(c, burst, step_cap) : 0);
+        if (has && (!c.active || (step_cap != 0 && c.steps >= step_cap))) {
+            store_cand(s, c);
+            has = false;
         }
         bool stop = false;
         if (lane == 0) stop = global_ns() - t0 > budget_ns;

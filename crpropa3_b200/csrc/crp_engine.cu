@@ -225,8 +225,24 @@ crp_status validate_module(const crp_module_desc &m) {
     return CRP_OK;
 }
 
+// The pair records of a Grid3f: 32 bytes per cell, {x, y, z, 0} of the cell and
+// of its upper neighbour in z (periodic).  A trilinear gather is then four
+// aligned 256-bit loads, one sector each, where the packed cells took 24
+// scalar loads and cells padded to 16 bytes eight 128-bit ones (six sectors on
+// average).  Grids above 2^30 cells (34 GB of records) are read packed.
+constexpr size_t kPairCells = (size_t)1 << 30;
+
+__global__ void pair_records_kernel(const float *g, unsigned nz, unsigned cells, float4 *pairs) {
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= cells) return;
+    const unsigned j = i % nz == nz - 1 ? i - (nz - 1) : i + 1;
+    const float *a = g + 3 * (size_t)i, *b = g + 3 * (size_t)j;
+    pairs[2 * (size_t)i] = make_float4(__ldg(a), __ldg(a + 1), __ldg(a + 2), 0.f);
+    pairs[2 * (size_t)i + 1] = make_float4(__ldg(b), __ldg(b + 1), __ldg(b + 2), 0.f);
+}
+
 // A Grid3f (comps 3) or Grid1f (comps 1) on the device: the cell values, the
-// padded copy of a Grid3f for the mixed form, and GridProperties (Grid.h:75).
+// pair records of a Grid3f, and GridProperties (Grid.h:75).
 crp_status build_grid(crp_plan *p, const crp_grid3f_desc &g, int comps, DevGrid &dg) {
     const char *name = comps == 3 ? "Grid3f" : "Grid1f";
     if (!g.values || g.nx == 0 || g.ny == 0 || g.nz == 0)
@@ -238,14 +254,22 @@ crp_status build_grid(crp_plan *p, const crp_grid3f_desc &g, int comps, DevGrid 
     size_t cells = (size_t)g.nx * g.ny * g.nz;
     crp_status st = upload(p, g.values, cells * comps, &dg.values);
     if (st) return st;
-    dg.values4 = nullptr;
-    if (comps == 3 && p->precision == CRP_PRECISION_MIXED) {
-        // 16-byte cells: one aligned 128-bit load per corner
-        std::vector<float4> pad(cells);
-        for (size_t i = 0; i < cells; i++)
-            pad[i] = make_float4(g.values[3 * i], g.values[3 * i + 1], g.values[3 * i + 2], 0.f);
-        st = upload(p, pad.data(), cells, &dg.values4);
-        if (st) return st;
+    dg.pairs = nullptr;
+    if (comps == 3 && cells <= kPairCells) {
+        void *d = nullptr;
+        const cudaError_t e = cudaMalloc(&d, cells * 32);
+        if (e == cudaSuccess) {
+            p->owned.push_back(d);
+            pair_records_kernel<<<(unsigned)((cells + 255) / 256), 256>>>(dg.values, (unsigned)g.nz, (unsigned)cells,
+                                                                          static_cast<float4 *>(d));
+            CUDA_TRY(cudaGetLastError());
+            CUDA_TRY(cudaStreamSynchronize(0));  // runs may use any stream
+            dg.pairs = static_cast<const float *>(d);
+        } else if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();  // too large beside the grid: the packed values are read
+        } else {
+            return cuda_fail(e, "cudaMalloc(pair records)");
+        }
     }
     dg.nx = (int)g.nx; dg.ny = (int)g.ny; dg.nz = (int)g.nz;
     dg.reflective = g.reflective;
@@ -626,6 +650,11 @@ crp_status crp_plan_create(const crp_plan_desc *desc, crp_plan **out) {
         crp_status st = build_component(p, desc->fields[i], d.fields[i]);
         if (st) { delete p; return st; }
     }
+    d.dev_fields = nullptr;
+    if (d.n_fields > 0) {
+        crp_status st = upload(p, d.fields, (size_t)d.n_fields, &d.dev_fields);
+        if (st) { delete p; return st; }
+    }
     int nfeat_total = 0;
     for (int i = 0; i < desc->n_modules; i++) {
         const crp_module_desc &m = desc->modules[i];
@@ -678,10 +707,9 @@ crp_status crp_plan_create(const crp_plan_desc *desc, crp_plan **out) {
     }
     if (d.n_fields == 1 && !desc->fields[0].periodic && desc->fields[0].kind == CRP_FIELD_GRID) {
         const DevGrid &g = d.fields[0].grid;
-        const bool padded = p->precision != CRP_PRECISION_MIXED || g.values4 != nullptr;
-        const bool small = (uint64_t)g.nx * g.ny * g.nz < (1ull << 31);  // 32-bit cell indices
+        const bool small = g.pairs != nullptr;  // at most 2^30 cells: 32-bit cell indices
         const bool trilinear = g.interp == CRP_INTERPOLATION_TRILINEAR;
-        p->fs = (!g.reflective && !g.clip_volume && g.pow2 && padded && small && trilinear) ? FS_GRID_PERIODIC
+        p->fs = (!g.reflective && !g.clip_volume && g.pow2 && small && trilinear) ? FS_GRID_PERIODIC
                                                                                            : FS_GRID;
     }
     else if (d.n_fields == 1 && !desc->fields[0].periodic && desc->fields[0].kind == CRP_FIELD_PLANE_WAVE)
@@ -1058,10 +1086,11 @@ static crp_status run_device(crp_plan *p, const crp_candidates *c, uint64_t n, c
             if (ls) return ls;
             launches++;  // the key kernel (the radix sort is CUB's)
         }
+        const int lanes = lanes_per_warp(n_threads, p->num_sms, kSpreadWarpsPerSm);
         auto step = [&](uint64_t nt, const uint32_t *li, cudaStream_t ss) {
             return (p->precision == CRP_PRECISION_FP64)
-                ? launch_fp64_chunk(p->dev, s, nt, spl, o.max_steps, p->d_cnt, rec, li, list_out, p->fs, block, ss)
-                : launch_mixed_chunk(p->dev, s, nt, spl, o.max_steps, p->d_cnt, rec, li, list_out, p->fs, block, ss);
+                ? launch_fp64_chunk(p->dev, s, nt, spl, o.max_steps, p->d_cnt, rec, li, list_out, p->fs, block, lanes, ss)
+                : launch_mixed_chunk(p->dev, s, nt, spl, o.max_steps, p->d_cnt, rec, li, list_out, p->fs, block, lanes, ss);
         };
         cudaError_t e = cudaSuccess;
         if (in && !list_in) {

@@ -16,7 +16,8 @@ constexpr int kMaxFeatures = 8;  // observer features of all modules of a plan
 
 struct DevGrid {
     const float *values;   // packed Vector3f cells, 12 B each (Grid.h:338 order)
-    const float4 *values4; // the same cells padded to 16 B (mixed form), or null
+    const float *pairs;    // pair records: per cell 32 B {x, y, z, 0} of the cell and of its upper
+                           // (periodic) z neighbour, or null
     int nx, ny, nz;
     int reflective;
     int clip_volume;
@@ -174,6 +175,7 @@ struct DevPlan {
     int shape;       // ChainShape (chain.cuh) the module sequence matches
     uint64_t seed;
     DevComponent fields[kMaxFields];
+    const DevComponent *dev_fields;  // device copy of the n_fields components (field_sum)
     DevModule modules[kMaxModules];
     DevFeature feat[kMaxFeatures];
 };

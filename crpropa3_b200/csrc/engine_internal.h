@@ -16,7 +16,7 @@ enum FieldSig {
     FS_GRID = 1,       // one MagneticFieldGrid, not wrapped
     FS_PLANE_WAVE = 2, // one PlaneWaveTurbulence, not wrapped
     FS_GRID_PERIODIC = 3  // FS_GRID with a periodic grid of power-of-two dimensions, no
-                          // clipVolume (and the padded copy, mixed form): no runtime checks
+                          // clipVolume and with pair records: no runtime checks
 };
 
 // Persistent stepping launch (chain.cuh persistent_body): `grid` CTAs of 128
@@ -35,14 +35,29 @@ struct PersistentArgs {
     uint64_t step_cap;
 };
 
+// Candidates per warp of a chunked launch of n candidates.  A launch that
+// cannot give every scheduler of the GPU a full warp (four per SM) spreads its
+// candidates over one warp per scheduler instead: its run time is the slowest
+// warp's chain of dependent instructions, and a warp with fewer candidates
+// makes fewer passes for lanes that diverge (retries, cell changes, early ends).
+// More warps than that share a scheduler and lose again (10^4 Cash-Karp
+// candidates, FP64, 64^3 grid: 7.8 ms at 32 per warp, 6.9 ms at 4 warps per SM,
+// 7.2 ms at 8; 10^5 nuclei: 71.3 ms at 4, 73.1 ms at 8).
+constexpr int kSpreadWarpsPerSm = 4;
+inline int lanes_per_warp(uint64_t n, int num_sms, int warps_per_sm) {
+    const uint64_t warps = (uint64_t)num_sms * (uint64_t)warps_per_sm;
+    const uint64_t l = (n + warps - 1) / warps;
+    return l < 1 ? 1 : l > 32 ? 32 : (int)l;
+}
+
 // step_fp64.cu
-// One launch of the chunked stepping kernel: threads t < n advance candidate
-// perm[t] (t without perm) by at most max_steps chain iterations; candidates
-// still active afterwards are appended to perm_out (may be null) and counted
-// in cnt->active_left.
+// One launch of the chunked stepping kernel: slots t < n (`lanes` of them per
+// warp) advance candidate perm[t] (t without perm) by at most max_steps chain
+// iterations; candidates still active afterwards are appended to perm_out
+// (may be null) and counted in cnt->active_left.
 cudaError_t launch_fp64_chunk(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
                               uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
-                              const uint32_t *perm, uint32_t *perm_out, int fs, int block,
+                              const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
                               cudaStream_t st);
 cudaError_t launch_fp64_field(const DevPlan &P, uint64_t n, const double *pos, double *out,
                               cudaStream_t st);
@@ -53,13 +68,34 @@ cudaError_t launch_fp64_persistent(const DevPlan &P, const DevState &s, const Pe
 // step_mixed.cu
 cudaError_t launch_mixed_chunk(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
                                uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
-                               const uint32_t *perm, uint32_t *perm_out, int fs, int block,
+                               const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
                                cudaStream_t st);
-// step_mixed_bp.cu: the Boris-push part of launch_mixed_chunk
+// step_fp64_bp.cu, step_fp64_ck.cu, step_mixed_bp.cu, step_mixed_ck.cu: the
+// Boris-push and Cash-Karp parts of the launchers above and below
+cudaError_t launch_fp64_bp_chunk(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
+                                  uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
+                                  const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
+                                  cudaStream_t st);
+cudaError_t launch_fp64_bp_persistent(const DevPlan &P, const DevState &s, const PersistentArgs &a,
+                                DevCounters *cnt, const DevRecords &rec, int fs, int grid, cudaStream_t st);
+cudaError_t launch_fp64_ck_chunk(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
+                                  uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
+                                  const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
+                                  cudaStream_t st);
+cudaError_t launch_fp64_ck_persistent(const DevPlan &P, const DevState &s, const PersistentArgs &a,
+                                DevCounters *cnt, const DevRecords &rec, int fs, int grid, cudaStream_t st);
 cudaError_t launch_mixed_bp_chunk(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
                                   uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
-                                  const uint32_t *perm, uint32_t *perm_out, int fs, int block,
+                                  const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
                                   cudaStream_t st);
+cudaError_t launch_mixed_bp_persistent(const DevPlan &P, const DevState &s, const PersistentArgs &a,
+                                DevCounters *cnt, const DevRecords &rec, int fs, int grid, cudaStream_t st);
+cudaError_t launch_mixed_ck_chunk(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
+                                  uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
+                                  const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
+                                  cudaStream_t st);
+cudaError_t launch_mixed_ck_persistent(const DevPlan &P, const DevState &s, const PersistentArgs &a,
+                                DevCounters *cnt, const DevRecords &rec, int fs, int grid, cudaStream_t st);
 cudaError_t launch_mixed_persistent(const DevPlan &P, const DevState &s, const PersistentArgs &a,
                                     DevCounters *cnt, const DevRecords &rec, int fs, int grid,
                                     cudaStream_t st);

@@ -36,6 +36,13 @@
 #ifndef CRP_BP_FIXED_MIN_BLOCKS
 #define CRP_BP_FIXED_MIN_BLOCKS 6
 #endif
+// The general grid's code (clipVolume, reflection, other interpolations) needs
+// more registers: 4 blocks (300 000 candidates x 1000 steps over a 100^3 grid:
+// mixed 6.4 ms, FP64 12.6 ms; at 5 blocks 6.9 and 13.2; at 6 with spills 10.5
+// and 15.3).
+#ifndef CRP_BP_GRID_MIN_BLOCKS
+#define CRP_BP_GRID_MIN_BLOCKS 4
+#endif
 #ifndef CRP_CK_MIN_BLOCKS
 #define CRP_CK_MIN_BLOCKS 3
 #endif
@@ -52,9 +59,14 @@ __device__ __forceinline__ float dot(f3 a, f3 b) { return fmaf(a.x, b.x, fmaf(a.
 __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
 __device__ __forceinline__ double clipd(double x, double lo, double hi) { return dmax(lo, dmin(x, hi)); }
+// |v|^2 with its multiply-adds written out (see component_position)
+__device__ __forceinline__ double norm2(double x, double y, double z) { return fma(z, z, fma(x, x, __dmul_rn(y, y))); }
 
 __device__ __forceinline__ int wrap(int i, int n, bool pow2) {
-    return pow2 ? (i & (n - 1)) : (((i % n) + n) % n);
+    if (pow2) return i & (n - 1);
+    if ((unsigned)i < (unsigned)n) return i;  // inside the grid: no division
+    const int r = i % n;
+    return r < 0 ? r + n : r;
 }
 
 // Trilinear Grid3f interpolation: FP64 cell coordinates, FP32 weights and
@@ -69,31 +81,26 @@ __device__ __forceinline__ int wrap(int i, int n, bool pow2) {
 // the cache.
 struct CellFrac { float fx0, fy0, fz0; };
 
-__device__ __forceinline__ CellFrac grid_cell_load(const DevGrid &g, double x, double y, double z, Cand &cc) {
+__device__ __forceinline__ CellFrac grid_cell_load(const DevGrid &g, double x, double y, double z, unsigned &tag,
+                                                   float (&corner)[8][3]) {
     const double rx = (x - g.gox) * g.inv_sx, ry = (y - g.goy) * g.inv_sy, rz = (z - g.goz) * g.inv_sz;
-    const double flx = floor(rx), fly = floor(ry), flz = floor(rz);
-    const CellFrac f{(float)(rx - flx), (float)(ry - fly), (float)(rz - flz)};
-    const int ix0 = wrap((int)flx, g.nx, true), ix1 = (ix0 + 1 == g.nx) ? 0 : ix0 + 1;
-    const int iy0 = wrap((int)fly, g.ny, true), iy1 = (iy0 + 1 == g.ny) ? 0 : iy0 + 1;
-    const int iz0 = wrap((int)flz, g.nz, true), iz1 = (iz0 + 1 == g.nz) ? 0 : iz0 + 1;
-    // 32-bit cell indices (fewer than 2^31 cells)
+    const CellIndex c = cell_index(rx, ry, rz);
+    const CellFrac f{(float)__dsub_rn(rx, c.flx), (float)__dsub_rn(ry, c.fly), (float)__dsub_rn(rz, c.flz)};
+    // 32-bit cell indices (fewer than 2^31 cells); on a periodic grid the
+    // lower corner's index names the cell
     const unsigned sy = (unsigned)g.nz, sx = (unsigned)g.ny * (unsigned)g.nz;
-    const unsigned b00 = (unsigned)ix0 * sx + (unsigned)iy0 * sy, b10 = (unsigned)ix1 * sx + (unsigned)iy0 * sy;
-    const unsigned b01 = (unsigned)ix0 * sx + (unsigned)iy1 * sy, b11 = (unsigned)ix1 * sx + (unsigned)iy1 * sy;
-    const unsigned idx[8] = {b00 + iz0, b10 + iz0, b01 + iz0, b00 + iz1, b10 + iz1, b01 + iz1, b11 + iz0, b11 + iz1};
-    const long long k0 = (long long)idx[0], k7 = (long long)idx[7];
-    if (k0 != cc.cell0 || k7 != cc.cell7) {
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const float4 v = __ldg(g.values4 + idx[k]);
-            cc.corner[k][0] = v.x; cc.corner[k][1] = v.y; cc.corner[k][2] = v.z;
-        }
-        cc.cell0 = k0; cc.cell7 = k7;
+    const int ix0 = c.ix & (g.nx - 1), iy0 = c.iy & (g.ny - 1), iz0 = c.iz & (g.nz - 1);
+    const unsigned b00 = (unsigned)ix0 * sx + (unsigned)iy0 * sy;
+    if (b00 + iz0 != tag) {
+        const unsigned x1 = (unsigned)((ix0 + 1) & (g.nx - 1)) * sx, y1 = (unsigned)((iy0 + 1) & (g.ny - 1)) * sy;
+        const unsigned x0 = (unsigned)ix0 * sx, y0 = (unsigned)iy0 * sy;
+        load_corner_pairs<true>(g.pairs, b00, x1 + y0, x0 + y1, x1 + y1, iz0, corner);
+        tag = b00 + iz0;
     }
     return f;
 }
 
-__device__ __forceinline__ f3 grid_cell_interp(const CellFrac &f, const Cand &cc) {
+__device__ __forceinline__ f3 grid_cell_interp(const CellFrac &f, const float (&corner)[8][3]) {
     const float fx0 = f.fx0, fy0 = f.fy0, fz0 = f.fz0;
     const float fx1 = 1.f - fx0, fy1 = 1.f - fy0, fz1 = 1.f - fz0;
     const float w[8] = {fx1 * fy1 * fz1, fx0 * fy1 * fz1, fx1 * fy0 * fz1, fx1 * fy1 * fz0,
@@ -101,16 +108,23 @@ __device__ __forceinline__ f3 grid_cell_interp(const CellFrac &f, const Cand &cc
     float bx = 0.f, by = 0.f, bz = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        bx = fmaf(cc.corner[k][0], w[k], bx);
-        by = fmaf(cc.corner[k][1], w[k], by);
-        bz = fmaf(cc.corner[k][2], w[k], bz);
+        bx = fmaf(corner[k][0], w[k], bx);
+        by = fmaf(corner[k][1], w[k], by);
+        bz = fmaf(corner[k][2], w[k], bz);
     }
     return f3mk(bx, by, bz);
 }
 
-template <bool CACHE, bool PER = false>
+// FUSED: the cell fraction from the unrounded product of position and inverse
+// spacing (one multiply-add), as the fixed-step Boris kernels over any grid
+// form it; otherwise from the rounded coordinate.  Written out so that it does
+// not depend on how the compiler contracts the expression in each kernel.
+template <bool CACHE, bool PER = false, bool FUSED = false>
 __device__ __forceinline__ f3 grid_field_t(const DevGrid &g, double x, double y, double z, Cand *cc) {
-    if (CACHE && PER) return grid_cell_interp(grid_cell_load(g, x, y, z, *cc), *cc);
+    if (CACHE && PER) {
+        const CellFrac f = grid_cell_load(g, x, y, z, cc->tag, cc->corner);
+        return grid_cell_interp(f, cc->corner);
+    }
     if (!PER && g.interp != CRP_INTERPOLATION_TRILINEAR) {  // tricubic, nearest (Grid.h:328-331)
         const gi3 v = gi_vector_other(g, x, y, z);
         return f3mk(v.x, v.y, v.z);
@@ -121,7 +135,16 @@ __device__ __forceinline__ f3 grid_field_t(const DevGrid &g, double x, double y,
     }
     double rx = (x - g.gox) * g.inv_sx, ry = (y - g.goy) * g.inv_sy, rz = (z - g.goz) * g.inv_sz;
     double flx = floor(rx), fly = floor(ry), flz = floor(rz);
-    float fx0 = (float)(rx - flx), fy0 = (float)(ry - fly), fz0 = (float)(rz - flz);
+    float fx0, fy0, fz0;
+    if (FUSED) {
+        fx0 = (float)fma(x - g.gox, g.inv_sx, -flx);
+        fy0 = (float)fma(y - g.goy, g.inv_sy, -fly);
+        fz0 = (float)fma(z - g.goz, g.inv_sz, -flz);
+    } else {
+        fx0 = (float)__dsub_rn(rx, flx);
+        fy0 = (float)__dsub_rn(ry, fly);
+        fz0 = (float)__dsub_rn(rz, flz);
+    }
     int ix0, ix1, iy0, iy1, iz0, iz1;
     if (!PER && g.reflective) {
         double r[3] = {rx, ry, rz};
@@ -162,11 +185,11 @@ __device__ __forceinline__ f3 grid_field_t(const DevGrid &g, double x, double y,
     float (*c)[3] = CACHE ? cc->corner : lc;
     const long long k0 = (long long)idx[0], k7 = (long long)idx[7];
     if (!CACHE || k0 != cc->cell0 || k7 != cc->cell7) {
-        if (PER || g.values4) {
+        if (PER || g.pairs) {
+            load_corner_pairs<CACHE>(g.pairs, b00, b10, b01, b11, iz0, c);
+            if (!PER && iz1 == iz0) {  // the reflective edge: no upper neighbour
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                float4 v = __ldg(g.values4 + idx[k]);
-                c[k][0] = v.x; c[k][1] = v.y; c[k][2] = v.z;
+                for (int a = 0; a < 3; a++) { c[3][a] = c[0][a]; c[4][a] = c[1][a]; c[5][a] = c[2][a]; c[7][a] = c[6][a]; }
             }
         } else {
 #pragma unroll
@@ -956,22 +979,31 @@ __device__ __forceinline__ f3 component_field(const DevComponent &f, double x, d
     }
 }
 
+// The field of any list of components.  Not inlined: the Cash-Karp step
+// evaluates the field six times and the adaptive Boris push three times, and
+// with the body of every field class inlined at each the kernels waited for
+// instructions (no_instruction 1.4-1.6 cycles per issued one).
 // sh: the plan's plane-wave table staged in shared memory (at most one
 // plane-wave component), or null.
-template <int FS>
-__device__ __forceinline__ f3 field_at(const DevPlan &P, double x, double y, double z,
-                                       Cand *cc = nullptr, const PwTab *sh = nullptr) {
-    if (FS == FS_GRID) return grid_field_t<true>(P.fields[0].grid, x, y, z, cc);
-    if (FS == FS_GRID_PERIODIC) return grid_field_t<true, true>(P.fields[0].grid, x, y, z, cc);
-    if (FS == FS_PLANE_WAVE) return plane_wave_field(P.fields[0].pw, x, y, z, sh);
-    if (P.n_fields == 1) return component_field(P.fields[0], x, y, z, sh);
+// The components are read from device memory (uniform addresses, L1 hits).
+__device__ __noinline__ f3 field_sum(const DevComponent *f, int n, double x, double y, double z, const PwTab *sh) {
+    if (n == 1) return component_field(f[0], x, y, z, sh);
     f3 b = f3mk(0.f, 0.f, 0.f);
 #pragma unroll 1
-    for (int i = 0; i < P.n_fields; i++) {
-        f3 c = component_field(P.fields[i], x, y, z, sh);
+    for (int i = 0; i < n; i++) {
+        f3 c = component_field(f[i], x, y, z, sh);
         b.x += c.x; b.y += c.y; b.z += c.z;
     }
     return b;
+}
+
+template <int FS, bool FUSED = false>
+__device__ __forceinline__ f3 field_at(const DevPlan &P, double x, double y, double z,
+                                       Cand *cc = nullptr, const PwTab *sh = nullptr) {
+    if (FS == FS_GRID) return grid_field_t<true, false, FUSED>(P.fields[0].grid, x, y, z, cc);
+    if (FS == FS_GRID_PERIODIC) return grid_field_t<true, true>(P.fields[0].grid, x, y, z, cc);
+    if (FS == FS_PLANE_WAVE) return plane_wave_field(P.fields[0].pw, x, y, z, sh);
+    return field_sum(P.dev_fields, P.n_fields, x, y, z, sh);
 }
 
 // Candidate::setCurrentStep (Candidate.cpp:92): the time increment s / c is
@@ -1009,73 +1041,89 @@ __device__ __forceinline__ void bp_rotate_drift(double &x, double &y, double &z,
     x = fma(ux, hh, x); y = fma(uy, hh, y); z = fma(uz, hh, z);
 }
 
+// t = B * q / 2 / m * step / c with m = E/c^2  ->  B * (q c step / (2 E)); the
+// factor of B and the step, formed in FP32 like the rotation it scales.
+__device__ __forceinline__ float boris_kq(double q, double E) {
+    return __fdividef((float)(q * (0.5 * kCLight)), (float)E);
+}
+
+// The step of a neutral candidate (PropagationBP.cpp:67, PropagationCK.cpp:81).
+__device__ __forceinline__ void neutral_step(const DevModule &m, Cand &c) {
+    const double step = clipd(c.next, m.min_step, m.max_step);
+    c.x = fma(c.dx, step, c.x); c.y = fma(c.dy, step, c.y); c.z = fma(c.dz, step, c.z);
+    set_current_step(c, step);
+    c.next = m.max_step;
+}
+
 // One PropagationBP::dY (PropagationBP.cpp:19) with FP32 rotation increment.
-template <int FS>
+template <int FS, bool FUSED>
 __device__ __forceinline__ void bp_dy(const DevPlan &P, double &x, double &y, double &z, double &ux,
                                       double &uy, double &uz, double step, float kt, Cand *cc) {
     double hh = 0.5 * step;
     x = fma(ux, hh, x); y = fma(uy, hh, y); z = fma(uz, hh, z);
-    f3 B = field_at<FS>(P, x, y, z, cc);
+    f3 B = field_at<FS, FUSED>(P, x, y, z, cc);
     bp_rotate_drift(x, y, z, ux, uy, uz, B, kt, hh);
 }
 
 template <int FS, int MODE = 0>
 struct BP {
     static constexpr bool kReadsStepCount = false;
-    __device__ static void process(const DevPlan &P, const DevModule &m, Cand &c, StepCount &sc) {
+    static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
+    struct Try {
+        double step;
+        int guard;
+    };
+    // Start of PropagationBP::process; false when the step is done (neutral).
+    __device__ __forceinline__ static bool begin(const DevPlan &P, const DevModule &m, Cand &c, Try &t) {
         c.px = c.x; c.py = c.y; c.pz = c.z;
-        double q = c.q, step = m.max_step;
-        if (q == 0) {
-            step = clipd(c.next, m.min_step, m.max_step);
-            c.x = fma(c.dx, step, c.x); c.y = fma(c.dy, step, c.y); c.z = fma(c.dz, step, c.z);
-            set_current_step(c, step);
-            c.next = m.max_step;
-            return;
+        if (c.q == 0) {
+            neutral_step(m, c);
+            return false;
         }
-        double newStep = step;
-        // t = B * q / 2 / m * step / c with m = E/c^2  ->  B * (q c step / (2 E)),
-        // formed in FP32 like the rotation it scales
-        const float kq = __fdividef((float)(q * (0.5 * kCLight)), (float)c.E);
+        t.step = MODE == 1 ? m.max_step : clipd(c.next, m.min_step, m.max_step);
+        t.guard = 0;
+        return true;
+    }
+    // One try; true when the step is done.
+    __device__ __forceinline__ static bool attempt(const DevPlan &P, const DevModule &m, Cand &c, Try &t,
+                                                   StepCount &sc) {
+        double step = t.step, newStep = step;
+        const float kq = boris_kq(c.q, c.E);
         double xo = c.x, yo = c.y, zo = c.z, uxo = c.dx, uyo = c.dy, uzo = c.dz;
-        if (MODE == 1 || (MODE == 0 && m.min_step == m.max_step)) {
-            bp_dy<FS>(P, xo, yo, zo, uxo, uyo, uzo, step, kq * (float)step, &c);
+        if (MODE == 1) {
+            bp_dy<FS, true>(P, xo, yo, zo, uxo, uyo, uzo, step, kq * (float)step, &c);
             sc.tries++; sc.evals++;
         } else {
-            step = clipd(c.next, m.min_step, m.max_step);
-            newStep = step;
-            for (int guard = 0; guard < 4096; guard++) {
-                double x1 = c.x, y1 = c.y, z1 = c.z, u1x = c.dx, u1y = c.dy, u1z = c.dz;
-                double x2 = c.x, y2 = c.y, z2 = c.z, u2x = c.dx, u2y = c.dy, u2z = c.dz;
-                const float kts = kq * (float)step;
-                bp_dy<FS>(P, x1, y1, z1, u1x, u1y, u1z, step, kts, &c);
-                bp_dy<FS>(P, x2, y2, z2, u2x, u2y, u2z, step / 2, 0.5f * kts, &c);
-                bp_dy<FS>(P, x2, y2, z2, u2x, u2y, u2z, step / 2, 0.5f * kts, &c);
-                sc.tries++; sc.evals += 3;
-                double ex = x1 - x2, ey = y1 - y2, ez = z1 - z2;
-                double S = sqrt(ex * ex + ey * ey + ez * ez) / (step * 0.75);
-                xo = x1; yo = y1; zo = z1; uxo = u1x; uyo = u1y; uzo = u1z;
-                double r = sqrt(3.0 * S * S) / m.tolerance;
-                if (r > 1) {
-                    if (step == m.min_step) break;
-                    newStep = step * 0.95 * pow(r, -0.2);
-                    newStep = dmax(newStep, 0.1 * step);
-                    newStep = dmax(newStep, m.min_step);
-                    step = newStep;
-                } else {
-                    if (step != m.max_step) {
-                        newStep = step * 0.95 * pow(r, -0.2);
-                        newStep = dmin(newStep, 5 * step);
-                        newStep = dmin(newStep, m.max_step);
-                    }
-                    break;
+            // the full step, then two half steps: one loop body for the three
+            double x = c.x, y = c.y, z = c.z, ux = c.dx, uy = c.dy, uz = c.dz, h = step;
+            const float kts = kq * (float)step;
+            float kt = kts;
+#pragma unroll 1
+            for (int i = 0; i < 3; i++) {
+                bp_dy<FS, false>(P, x, y, z, ux, uy, uz, h, kt, &c);
+                if (i == 0) {
+                    xo = x; yo = y; zo = z; uxo = ux; uyo = uy; uzo = uz;
+                    x = c.x; y = c.y; z = c.z; ux = c.dx; uy = c.dy; uz = c.dz;
+                    h = step / 2;
+                    kt = 0.5f * kts;
                 }
             }
+            sc.tries++; sc.evals += 3;
+            double ex = xo - x, ey = yo - y, ez = zo - z;
+            double S = sqrt(norm2(ex, ey, ez)) / (step * 0.75);
+            double r = sqrt(3.0 * S * S) / m.tolerance;
+            if (step_control(m, r, step, newStep, [](double a, double b) { return pow(a, b); }) && ++t.guard < 4096) {
+                t.step = newStep;
+                return false;
+            }
+            if (t.guard == 4096) step = newStep;
         }
         renorm(uxo, uyo, uzo);
         c.x = xo; c.y = yo; c.z = zo;
         c.dx = uxo; c.dy = uyo; c.dz = uzo;
         set_current_step(c, step);
         c.next = newStep;
+        return true;
     }
 };
 
@@ -1093,10 +1141,11 @@ __constant__ double ck_eb[6] = {37. / 378. - 2825. / 27648., 0. - 0., 250. / 621
 
 // One Cash-Karp try in time h (PropagationCK::tryStep): stage derivatives in
 // FP32, stage positions as FP64 base + FP32 offset, error sum in FP64.
-// Returns the position / direction increments and the direction error norm.
+// Gives the end position and the direction increment, returns the direction
+// error norm.
 template <int FS>
 __device__ __forceinline__ double ck_try(const DevPlan &P, Cand &c, double h, float qc2E,
-                                         double &ddx, double &ddy, double &ddz, double &dux,
+                                         double &xo, double &yo, double &zo, double &dux,
                                          double &duy, double &duz) {
     // stage derivative kx_i = c * unit(u_i) (as a unit vector, the factor c
     // is applied to the sums), ku_i = (q c / E) (v_i x B_i)
@@ -1127,59 +1176,52 @@ __device__ __forceinline__ double ck_try(const DevPlan &P, Cand &c, double h, fl
         double e = ck_eb[i] * h;
         eux = fma((double)ku[i].x, e, eux); euy = fma((double)ku[i].y, e, euy); euz = fma((double)ku[i].z, e, euz);
     }
-    ddx = (double)sxx * (h * kCLight); ddy = (double)sxy * (h * kCLight); ddz = (double)sxz * (h * kCLight);
+    const double tcd = __dmul_rn(h, kCLight);
+    xo = fma((double)sxx, tcd, c.x); yo = fma((double)sxy, tcd, c.y); zo = fma((double)sxz, tcd, c.z);
     dux = (double)(sux * hf); duy = (double)(suy * hf); duz = (double)(suz * hf);
-    return sqrt(eux * eux + euy * euy + euz * euz);
+    return sqrt(norm2(eux, euy, euz));
 }
 
 template <int FS, int MODE = 0>
 struct CK {
     static constexpr bool kReadsStepCount = false;
-    __device__ static void process(const DevPlan &P, const DevModule &m, Cand &c, StepCount &sc) {
+    static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
+    struct Try {
+        double step;
+        int guard;
+    };
+    __device__ __forceinline__ static bool begin(const DevPlan &P, const DevModule &m, Cand &c, Try &t) {
         c.px = c.x; c.py = c.y; c.pz = c.z;
-        double step = m.max_step;
         if (c.q == 0) {
-            step = clipd(c.next, m.min_step, m.max_step);
-            c.x = fma(c.dx, step, c.x); c.y = fma(c.dy, step, c.y); c.z = fma(c.dz, step, c.z);
-            set_current_step(c, step);
-            c.next = m.max_step;
-            return;
+            neutral_step(m, c);
+            return false;
         }
+        t.step = MODE == 1 ? m.max_step : clipd(c.next, m.min_step, m.max_step);
+        t.guard = 0;
+        return true;
+    }
+    __device__ __forceinline__ static bool attempt(const DevPlan &P, const DevModule &m, Cand &c, Try &t,
+                                                   StepCount &sc) {
+        double step = t.step, newStep = step;
         const float qc2E = __fdividef((float)(c.q * (kCLight * kCLight)), (float)c.E);
-        double ddx, ddy, ddz, dux, duy, duz;
-        double newStep = step;
-        if (MODE == 1 || (MODE == 0 && m.min_step == m.max_step)) {
-            ck_try<FS>(P, c, step * kInvCLight, qc2E, ddx, ddy, ddz, dux, duy, duz);
-            sc.tries++; sc.evals += 6;
-        } else {
-            step = clipd(c.next, m.min_step, m.max_step);
-            newStep = step;
-            for (int guard = 0; guard < 4096; guard++) {
-                double err = ck_try<FS>(P, c, step * kInvCLight, qc2E, ddx, ddy, ddz, dux, duy, duz);
-                sc.tries++; sc.evals += 6;
-                double r = err / m.tolerance;
-                if (r > 1) {
-                    if (step == m.min_step) break;
-                    newStep = step * 0.95 * pow(r, -0.2);
-                    newStep = dmax(newStep, 0.1 * step);
-                    newStep = dmax(newStep, m.min_step);
-                    step = newStep;
-                } else {
-                    if (step != m.max_step) {
-                        newStep = step * 0.95 * pow(r, -0.2);
-                        newStep = dmin(newStep, 5 * step);
-                        newStep = dmin(newStep, m.max_step);
-                    }
-                    break;
-                }
+        double xo, yo, zo, dux, duy, duz;
+        const double err = ck_try<FS>(P, c, step * kInvCLight, qc2E, xo, yo, zo, dux, duy, duz);
+        sc.tries++; sc.evals += 6;
+        if (MODE != 1) {
+            const double r = err / m.tolerance;
+            if (step_control(m, r, step, newStep, [](double a, double b) { return pow(a, b); }) && ++t.guard < 4096) {
+                t.step = newStep;
+                return false;
             }
+            if (t.guard == 4096) step = newStep;
         }
-        c.x += ddx; c.y += ddy; c.z += ddz;
+        c.x = xo; c.y = yo; c.z = zo;
         double ux = c.dx + dux, uy = c.dy + duy, uz = c.dz + duz;
-        double inv = 1.0 / sqrt(ux * ux + uy * uy + uz * uz);
+        double inv = 1.0 / sqrt(norm2(ux, uy, uz));
         c.dx = ux * inv; c.dy = uy * inv; c.dz = uz * inv;
         set_current_step(c, step);
         c.next = newStep;
+        return true;
     }
 };
 
@@ -1265,7 +1307,7 @@ __device__ __forceinline__ bool sde_co_begin(const DevPlan &P, const DevModule &
         sde_lin_prop(m, c.x, c.y, c.z, c.time, h, lx, ly, lz);
         c.x = fma(c.dx, h * kCLight, c.x + lx); c.y = fma(c.dy, h * kCLight, c.y + ly);
         c.z = fma(c.dz, h * kCLight, c.z + lz);
-        set_current_step(c, h * kCLight);
+        set_current_step(c, __dmul_rn(h, kCLight));
         c.next = m.max_step;
         return false;
     }
@@ -1298,7 +1340,7 @@ __device__ __forceinline__ void sde_co_finish(const DevPlan &P, const DevModule 
         } else {
             c.x = fma(c.dx, h * kCLight, c.x); c.y = fma(c.dy, h * kCLight, c.y); c.z = fma(c.dz, h * kCLight, c.z);
         }
-        set_current_step(c, h * kCLight);
+        set_current_step(c, __dmul_rn(h, kCLight));
         c.next = clipd(5 * h * kCLight, m.min_step, m.max_step);
         return;
     }
@@ -1342,7 +1384,7 @@ __device__ __forceinline__ void sde_co_finish(const DevPlan &P, const DevModule 
     double dn = 1.0 / sqrt(ddot(dx, dy, dz, dx, dy, dz));
     c.x = POx; c.y = POy; c.z = POz;
     c.dx = dx * dn; c.dy = dy * dn; c.dz = dz * dn;
-    set_current_step(c, h * kCLight);
+    set_current_step(c, __dmul_rn(h, kCLight));
     c.next = (co.stepNumber > 1) ? h / ((double)co.stepNumber * (double)co.stepNumber) * kCLight
                                  : 4 * h * kCLight;
 }
@@ -1412,25 +1454,18 @@ __device__ __forceinline__ bool sde_co_consume(const DevPlan &P, const DevModule
 template <int FS>
 struct SDE {
     static constexpr bool kReadsStepCount = true;  // the Philox counter
-    __device__ static void process(const DevPlan &P, const DevModule &m, Cand &c, StepCount &sc) {
+    static constexpr bool kRetries = false;
+    struct Try {};
+    __device__ __forceinline__ static bool begin(const DevPlan &, const DevModule &, Cand &, Try &) { return true; }
+    __device__ __forceinline__ static bool attempt(const DevPlan &P, const DevModule &m, Cand &c, Try &,
+                                                   StepCount &sc) {
         SdeCo co;
-        if (!sde_co_begin<FS>(P, m, c, co)) return;
+        if (!sde_co_begin<FS>(P, m, c, co)) return true;
         while (sde_co_consume(P, m, c, co, field_at<FS>(P, co.qx, co.qy, co.qz, &c), sc)) {
         }
+        return true;
     }
 };
-
-
-// The non-propagation modules mi in [from, to) of one chain iteration.
-__device__ __forceinline__ void chain_part(const DevPlan &P, Cand &c, const DevRecords &rec, int from, int to) {
-#pragma unroll 1
-    for (int mi = from; mi < to; mi++) {
-        const DevModule &m = P.modules[mi];
-        if (m.kind == CRP_MODULE_MAX_TRAJECTORY_LENGTH) max_trajectory_length(m, c, rec, mi);
-        else if (m.kind == CRP_MODULE_OBSERVER) observer(P, m, c, rec, mi);
-        else if (m.kind == CRP_MODULE_BOUNDARY) boundary(m, c, rec, mi);
-    }
-}
 
 // step-mode variants selected by the launcher from min_step == max_step, so
 // that a fixed-step kernel carries no adaptive-controller registers
@@ -1438,44 +1473,82 @@ template <int FS> using BPFixed = BP<FS, 1>;
 // resident blocks of 128 threads per SM the register budget is sized for:
 // the fixed-step Boris push is latency bound on its gathers and wants warps
 template <class T> struct MinBlocks { static constexpr int value = 1; };
-template <int FS, int MODE> struct MinBlocks<BP<FS, MODE>> { static constexpr int value = MODE == 1 ? CRP_BP_FIXED_MIN_BLOCKS : 1; };
+template <int FS, int MODE> struct MinBlocks<BP<FS, MODE>> {
+    static constexpr int value = MODE != 1 ? 1 : FS == FS_GRID ? CRP_BP_GRID_MIN_BLOCKS : CRP_BP_FIXED_MIN_BLOCKS;
+};
 template <int FS, int MODE> struct MinBlocks<CK<FS, MODE>> { static constexpr int value = CRP_CK_MIN_BLOCKS; };
 template <int FS> using BPAdaptive = BP<FS, 2>;
 template <int FS> using CKFixed = CK<FS, 1>;
 template <int FS> using CKAdaptive = CK<FS, 2>;
 
 template <template <int> class Prop, int FS, int CS>
-__global__ void __launch_bounds__(128, MinBlocks<Prop<FS>>::value) mixed_chunk_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n,
-                                                          int max_steps, uint64_t step_cap,
-                                                          DevCounters *cnt, DevRecords rec,
-                                                          const uint32_t *perm, uint32_t *perm_out) {
-    chunk_body<Prop<FS>, CS>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out);
+__global__ void __launch_bounds__(128, MinBlocks<Prop<FS>>::value)
+mixed_chunk_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, int lanes, int max_steps, uint64_t step_cap,
+                   DevCounters *cnt, DevRecords rec, const uint32_t *perm, uint32_t *perm_out) {
+    chunk_body<Prop<FS>, CS>(P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
+}
+
+template <template <int> class Prop, int FS, int CS>
+__global__ void __launch_bounds__(128, MinBlocks<Prop<FS>>::value) mixed_persistent_kernel(
+    const __grid_constant__ DevPlan P, DevState s, PersistentArgs a, DevCounters *cnt, DevRecords rec) {
+    // the queue is written only between launches (advance_kernel)
+    const DevQueue q = *a.q;
+    const uint32_t *pending_in = q.cur ? a.list_b : a.list_a;
+    uint32_t *pending_out = q.cur ? a.list_a : a.list_b;
+    persistent_body<Prop<FS>, CS>(P, s, pending_in, q.n_pending, q.main_base, q.n_main, pending_out,
+                              a.burst, a.refill, a.budget_ns, a.step_cap, cnt, rec);
+}
+
+// The kernel of a field signature and chain shape: compiled chain shapes for
+// the single-field signatures and, for the backtracking chain [propagation,
+// MaximumTrajectoryLength, Observer], the generic field sum; otherwise the
+// module list is walked.
+template <class F>
+void for_signature(int fs, int shape, F f) {
+    using std::integral_constant;
+    integral_constant<int, CS_PM> pm;
+    integral_constant<int, CS_PMO> pmo;
+    integral_constant<int, CS_GENERIC> any;
+    if (fs == FS_GRID_PERIODIC) {
+        integral_constant<int, FS_GRID_PERIODIC> s;
+        if (shape == CS_PM) f(s, pm);
+        else if (shape == CS_PMO) f(s, pmo);
+        else f(s, any);
+    } else if (fs == FS_GRID) {
+        f(integral_constant<int, FS_GRID>(), any);
+    } else if (fs == FS_PLANE_WAVE) {
+        integral_constant<int, FS_PLANE_WAVE> s;
+        if (shape == CS_PM) f(s, pm);
+        else if (shape == CS_PMO) f(s, pmo);
+        else f(s, any);
+    } else {
+        integral_constant<int, FS_GENERIC> s;
+        if (shape == CS_PMO) f(s, pmo);
+        else f(s, any);
+    }
 }
 
 template <template <int> class Prop>
 cudaError_t launch_prop(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
                         uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
-                        const uint32_t *perm, uint32_t *perm_out, int fs, int block,
+                        const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
                         cudaStream_t st) {
-    unsigned grid = (unsigned)((n + block - 1) / block);
-#define CRP_CHUNK(FSV, CSV) mixed_chunk_kernel<Prop, FSV, CSV><<<grid, block, 0, st>>>(P, s, n, max_steps, \
-        step_cap, cnt, rec, perm, perm_out)
-    // compiled chain shapes for the single-field signatures; the generic
-    // field sum walks the module list
-    if (fs == FS_GRID_PERIODIC) {
-        if (P.shape == CS_PM) CRP_CHUNK(FS_GRID_PERIODIC, CS_PM);
-        else if (P.shape == CS_PMO) CRP_CHUNK(FS_GRID_PERIODIC, CS_PMO);
-        else CRP_CHUNK(FS_GRID_PERIODIC, CS_GENERIC);
-    } else if (fs == FS_GRID) {
-        CRP_CHUNK(FS_GRID, CS_GENERIC);
-    } else if (fs == FS_PLANE_WAVE) {
-        if (P.shape == CS_PM) CRP_CHUNK(FS_PLANE_WAVE, CS_PM);
-        else if (P.shape == CS_PMO) CRP_CHUNK(FS_PLANE_WAVE, CS_PMO);
-        else CRP_CHUNK(FS_PLANE_WAVE, CS_GENERIC);
-    } else {
-        CRP_CHUNK(FS_GENERIC, CS_GENERIC);
-    }
-#undef CRP_CHUNK
+    const uint64_t slots = (uint64_t)(block / 32) * (uint64_t)lanes;
+    const unsigned grid = (unsigned)((n + slots - 1) / slots);
+    for_signature(fs, P.shape, [&](auto f, auto c) {
+        mixed_chunk_kernel<Prop, decltype(f)::value, decltype(c)::value><<<grid, block, 0, st>>>(
+            P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
+    });
+    return cudaGetLastError();
+}
+
+template <template <int> class Prop>
+cudaError_t launch_persistent_prop(const DevPlan &P, const DevState &s, const PersistentArgs &a,
+                                   DevCounters *cnt, const DevRecords &rec, int fs, int grid,
+                                   cudaStream_t st) {
+    for_signature(fs, P.shape, [&](auto f, auto c) {
+        mixed_persistent_kernel<Prop, decltype(f)::value, decltype(c)::value><<<grid, 128, 0, st>>>(P, s, a, cnt, rec);
+    });
     return cudaGetLastError();
 }
 

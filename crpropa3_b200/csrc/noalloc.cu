@@ -147,7 +147,7 @@ extern "C" crp_status crp_run_device_noalloc(const crp_noalloc_grid_bp_desc *d,
     f.kind = CRP_FIELD_GRID;
     DevGrid &g = f.grid;
     g.values = d->grid_values;
-    g.values4 = nullptr;
+    g.pairs = nullptr;
     g.nx = (int)d->nx; g.ny = (int)d->ny; g.nz = (int)d->nz;
     g.reflective = d->reflective;
     g.clip_volume = d->clip_volume;
@@ -189,11 +189,12 @@ extern "C" crp_status crp_run_device_noalloc(const crp_noalloc_grid_bp_desc *d,
     const uint32_t *list_in = nullptr;
     uint32_t *list_out = list_a;
     for (;;) {
+        const int lanes = 32;  // this path never queries the device
         cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(DevCounters), stm);
         if (e != cudaSuccess) return cuda_noalloc_fail(e, "clearing the scratch counters");
         e = (d->precision == CRP_PRECISION_FP64)
-            ? launch_fp64_chunk(P, s, n_threads, spl, 0, cnt, rec, list_in, list_out, FS_GRID, 128, stm)
-            : launch_mixed_chunk(P, s, n_threads, spl, 0, cnt, rec, list_in, list_out, FS_GRID, 128, stm);
+            ? launch_fp64_chunk(P, s, n_threads, spl, 0, cnt, rec, list_in, list_out, FS_GRID, 128, lanes, stm)
+            : launch_mixed_chunk(P, s, n_threads, spl, 0, cnt, rec, list_in, list_out, FS_GRID, 128, lanes, stm);
         if (e != cudaSuccess) return cuda_noalloc_fail(e, "stepping kernel launch");
         DevCounters h;
         e = cudaMemcpyAsync(&h, cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, stm);

@@ -13,9 +13,9 @@
 // accumulated error of 10^3-10^6 steps at the FP64 level of the increments'
 // relative error times their size.
 //
-// This unit holds the Cash-Karp, DiffusionSDE and generic kernels and
-// their launchers; the fixed-step and adaptive Boris kernels are in
-// step_mixed_bp.cu.
+// This unit holds the DiffusionSDE kernels, the field kernel and the
+// launchers; the Boris and Cash-Karp kernels are in step_mixed_bp.cu and
+// step_mixed_ck.cu.
 #include "mixed_device.cuh"
 
 namespace crp {
@@ -278,39 +278,6 @@ mixed_sde_batch_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n
     append_active(cnt, perm_out, still, (uint32_t)i);
 }
 
-template <template <int> class Prop, int FS, int CS>
-__global__ void __launch_bounds__(128, MinBlocks<Prop<FS>>::value) mixed_persistent_kernel(
-    const __grid_constant__ DevPlan P, DevState s, PersistentArgs a, DevCounters *cnt, DevRecords rec) {
-    // the queue is written only between launches (advance_kernel)
-    const DevQueue q = *a.q;
-    const uint32_t *pending_in = q.cur ? a.list_b : a.list_a;
-    uint32_t *pending_out = q.cur ? a.list_a : a.list_b;
-    persistent_body<Prop<FS>, CS>(P, s, pending_in, q.n_pending, q.main_base, q.n_main, pending_out,
-                              a.burst, a.refill, a.budget_ns, a.step_cap, cnt, rec);
-}
-
-template <template <int> class Prop>
-cudaError_t launch_persistent_prop(const DevPlan &P, const DevState &s, const PersistentArgs &a,
-                                   DevCounters *cnt, const DevRecords &rec, int fs, int grid,
-                                   cudaStream_t st) {
-#define CRP_PERSIST(FSV, CSV) mixed_persistent_kernel<Prop, FSV, CSV><<<grid, 128, 0, st>>>(P, s, a, cnt, rec)
-    if (fs == FS_GRID_PERIODIC) {
-        if (P.shape == CS_PM) CRP_PERSIST(FS_GRID_PERIODIC, CS_PM);
-        else if (P.shape == CS_PMO) CRP_PERSIST(FS_GRID_PERIODIC, CS_PMO);
-        else CRP_PERSIST(FS_GRID_PERIODIC, CS_GENERIC);
-    } else if (fs == FS_GRID) {
-        CRP_PERSIST(FS_GRID, CS_GENERIC);
-    } else if (fs == FS_PLANE_WAVE) {
-        if (P.shape == CS_PM) CRP_PERSIST(FS_PLANE_WAVE, CS_PM);
-        else if (P.shape == CS_PMO) CRP_PERSIST(FS_PLANE_WAVE, CS_PMO);
-        else CRP_PERSIST(FS_PLANE_WAVE, CS_GENERIC);
-    } else {
-        CRP_PERSIST(FS_GENERIC, CS_GENERIC);
-    }
-#undef CRP_PERSIST
-    return cudaGetLastError();
-}
-
 __global__ void mixed_field_kernel(const __grid_constant__ DevPlan P, uint64_t n, const double *pos, double *out) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -322,17 +289,14 @@ __global__ void mixed_field_kernel(const __grid_constant__ DevPlan P, uint64_t n
 
 cudaError_t launch_mixed_chunk(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
                               uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
-                              const uint32_t *perm, uint32_t *perm_out, int fs, int block,
+                              const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
                               cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     int prop = P.modules[P.prop_index].propagator;
-    const DevModule &pm = P.modules[P.prop_index];
-    const bool fixed = pm.min_step == pm.max_step;
-    if (prop == CRP_PROP_BP)  // step_mixed_bp.cu
-        return launch_mixed_bp_chunk(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, st);
+    if (prop == CRP_PROP_BP)
+        return launch_mixed_bp_chunk(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, lanes, st);
     if (prop == CRP_PROP_CK)
-        return fixed ? launch_prop<CKFixed>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, st)
-                     : launch_prop<CKAdaptive>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, st);
+        return launch_mixed_ck_chunk(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, lanes, st);
     if (block > 128) block = 128;
     const unsigned grid = (unsigned)((n + block - 1) / block);
     // stage the plane-wave table in shared memory when there is exactly one
@@ -382,14 +346,9 @@ cudaError_t launch_mixed_chunk(const DevPlan &P, const DevState &s, uint64_t n, 
 cudaError_t launch_mixed_persistent(const DevPlan &P, const DevState &s, const PersistentArgs &a,
                                    DevCounters *cnt, const DevRecords &rec, int fs, int grid,
                                    cudaStream_t st) {
-    const DevModule &pm = P.modules[P.prop_index];
-    const bool fixed = pm.min_step == pm.max_step;
-    if (pm.propagator == CRP_PROP_BP)
-        return fixed ? launch_persistent_prop<BPFixed>(P, s, a, cnt, rec, fs, grid, st)
-                     : launch_persistent_prop<BPAdaptive>(P, s, a, cnt, rec, fs, grid, st);
-    if (pm.propagator == CRP_PROP_CK)
-        return fixed ? launch_persistent_prop<CKFixed>(P, s, a, cnt, rec, fs, grid, st)
-                     : launch_persistent_prop<CKAdaptive>(P, s, a, cnt, rec, fs, grid, st);
+    const int prop = P.modules[P.prop_index].propagator;
+    if (prop == CRP_PROP_BP) return launch_mixed_bp_persistent(P, s, a, cnt, rec, fs, grid, st);
+    if (prop == CRP_PROP_CK) return launch_mixed_ck_persistent(P, s, a, cnt, rec, fs, grid, st);
     return launch_persistent_prop<SDE>(P, s, a, cnt, rec, fs, grid, st);
 }
 

@@ -1,0 +1,27 @@
+// step_mixed_ck.cu -- the mixed-precision Cash-Karp (PropagationCK) kernels: chunked
+// and persistent launches of the fixed-step and adaptive forms for every field
+// signature (the device code is in mixed_device.cuh).
+#include "mixed_device.cuh"
+
+namespace crp {
+
+cudaError_t launch_mixed_ck_chunk(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
+                                  uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
+                                  const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
+                                  cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    const DevModule &pm = P.modules[P.prop_index];
+    const bool fixed = pm.min_step == pm.max_step;
+    return fixed ? launch_prop<CKFixed>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, lanes, st)
+                 : launch_prop<CKAdaptive>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, lanes, st);
+}
+
+cudaError_t launch_mixed_ck_persistent(const DevPlan &P, const DevState &s, const PersistentArgs &a,
+                                       DevCounters *cnt, const DevRecords &rec, int fs, int grid, cudaStream_t st) {
+    const DevModule &pm = P.modules[P.prop_index];
+    const bool fixed = pm.min_step == pm.max_step;
+    return fixed ? launch_persistent_prop<CKFixed>(P, s, a, cnt, rec, fs, grid, st)
+                 : launch_persistent_prop<CKAdaptive>(P, s, a, cnt, rec, fs, grid, st);
+}
+
+}  // namespace crp
