@@ -531,6 +531,83 @@ __device__ __forceinline__ void chunk_body(const DevPlan &P, const DevState &s, 
     append_active(cnt, perm_out, still, (uint32_t)i);
 }
 
+// Chunked launch of the chain [fixed-step PropagationBP, MaximumTrajectoryLength]
+// (CS_PM) over a periodic power-of-two grid.  What the chain does besides the
+// push is known before the first step: the trajectory length and time after
+// every step are running sums of the step, so the number of steps this launch
+// makes is counted first (the same sums in the same order), and the loop over
+// them holds only position, direction and the cell's corners.  The previous
+// position is written where the last step begins, the other members after it.
+// Push: the push of one precision form; Push::sane(P, q, E): whether its
+// short forms hold for this candidate (else the chain is run as advance() runs
+// it).
+template <class Push, class Prop>
+__device__ __forceinline__ void boris_body(const DevPlan &P, const DevState &s, uint64_t n, int lanes, int max_steps,
+                                           uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
+                                           const uint32_t *perm_in, uint32_t *perm_out) {
+    const uint64_t t = candidate_slot(lanes, n);
+    StepCount sc;
+    int k = 0;
+    bool still = false;
+    uint64_t i = 0;
+    if (t < n) i = perm_in ? perm_in[t] : t;
+    if (t < n && s.active[i]) {
+        const DevModule &m = P.modules[0], &end = P.modules[1];
+        const double q = s.charge[i], E = s.energy[i];
+        if (!Push::sane(P, q, E)) {
+            Cand c;
+            load_cand(s, i, c);
+            k = advance<Prop, CS_PM>(P, c, rec, sc, launch_steps(c, max_steps, step_cap));
+            still = c.active && (step_cap == 0 || c.steps < step_cap);
+            store_cand(s, c);
+        } else {
+            const double step = m.max_step;
+            const double most = end.per_candidate ? (s.max_length ? s.max_length[i] : 0.0) : end.max_length;
+            const uint64_t before = s.steps ? s.steps[i] : 0;
+            double len = s.len[i], time = s.time[i];
+            int kmax = max_steps;
+            if (step_cap) {
+                const uint64_t left = step_cap > before ? step_cap - before : 0;
+                kmax = left < (uint64_t)max_steps ? (int)left : max_steps;
+            }
+            bool ended = false;
+            while (k < kmax && !ended) {
+                len += step;
+                time = Push::later(time, step);
+                ended = len >= most;
+                k++;
+            }
+            if (k > 0) {
+                Push push(P, q, E);
+                double x = s.x[i], y = s.y[i], z = s.z[i], ux = s.dx[i], uy = s.dy[i], uz = s.dz[i];
+                for (int j = k; j > 0; j--) {
+                    if (j == 1) { s.px[i] = x; s.py[i] = y; s.pz[i] = z; }
+                    push.step(P, x, y, z, ux, uy, uz);
+                }
+                sc.tries = sc.evals = (unsigned)k;
+                const double left = most - len;  // Candidate::limitNextStep (Candidate.cpp:102)
+                s.x[i] = x; s.y[i] = y; s.z[i] = z;
+                s.dx[i] = ux; s.dy[i] = uy; s.dz[i] = uz;
+                s.len[i] = len; s.time[i] = time; s.cur[i] = step;
+                s.next[i] = !ended && left < step ? left : step;
+                if (s.steps) s.steps[i] = before + (uint64_t)k;
+                if (ended) {  // MaximumTrajectoryLength rejects it
+                    if (end.record) {
+                        Cand c;
+                        load_cand(s, i, c);
+                        write_record(rec, c, 1);
+                    }
+                    s.flags[i] = s.flags[i] | CRP_FLAG_REJECTED;
+                    s.active[i] = 0;
+                }
+            }
+            still = !ended && (step_cap == 0 || before + (uint64_t)k < step_cap);
+        }
+    }
+    flush_counters(cnt, (unsigned long long)k, sc);
+    append_active(cnt, perm_out, still, (uint32_t)i);
+}
+
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

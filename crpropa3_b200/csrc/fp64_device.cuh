@@ -79,6 +79,44 @@ __device__ __forceinline__ int grid_wrap(int i, int n) {
 // PER: the grid is periodic with power-of-two dimensions and has no
 // clipVolume (FS_GRID_PERIODIC): those branches are compiled out and the
 // periodic clamp is a mask (equal to the double modulo of Grid.h:31 there).
+__device__ __forceinline__ d3 trilinear(const float (&c)[8][3], double fX0, double fY0, double fZ0) {
+    const float fx1 = (float)(1 - fX0), fy1 = (float)(1 - fY0), fz1 = (float)(1 - fZ0);
+    const float fx0 = (float)fX0, fy0 = (float)fY0, fz0 = (float)fZ0;
+    const float wx[8] = {fx1, fx0, fx1, fx1, fx0, fx1, fx0, fx0};
+    const float wy[8] = {fy1, fy1, fy0, fy1, fy1, fy0, fy0, fy0};
+    const float wz[8] = {fz1, fz1, fz1, fz0, fz0, fz0, fz1, fz0};
+    float bx = 0.f, by = 0.f, bz = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        bx += c[k][0] * wx[k] * wy[k] * wz[k];
+        by += c[k][1] * wx[k] * wy[k] * wz[k];
+        bz += c[k][2] * wx[k] * wy[k] * wz[k];
+    }
+    return mk(bx, by, bz);
+}
+
+// a / b rounded to nearest by a reciprocal, defined with the division-free push below.
+__device__ __forceinline__ double quotient(double a, double b, double rb);
+
+// The periodic power-of-two grid (PER below) with its own corner cache.  The
+// coordinates are quotients by the spacing (g.inv_s*: its correctly rounded
+// reciprocal); where one is too small for an exact remainder its cell and
+// single-precision fraction do not depend on the last bit.
+__device__ __forceinline__ d3 grid_periodic(const DevGrid &g, d3 pos, unsigned &tag, float (&corner)[8][3]) {
+    const double rx = quotient(pos.x - g.gox, g.sx, g.inv_sx), ry = quotient(pos.y - g.goy, g.sy, g.inv_sy),
+                 rz = quotient(pos.z - g.goz, g.sz, g.inv_sz);
+    const CellIndex i = cell_index(rx, ry, rz);
+    const unsigned sy = (unsigned)g.nz, sx = (unsigned)g.ny * (unsigned)g.nz;
+    const int ix0 = i.ix & (g.nx - 1), iy0 = i.iy & (g.ny - 1), iz0 = i.iz & (g.nz - 1);
+    const unsigned x0 = (unsigned)ix0 * sx, y0 = (unsigned)iy0 * sy;
+    if (x0 + y0 + iz0 != tag) {
+        const unsigned x1 = (unsigned)((ix0 + 1) & (g.nx - 1)) * sx, y1 = (unsigned)((iy0 + 1) & (g.ny - 1)) * sy;
+        load_corner_pairs<true>(g.pairs, x0 + y0, x1 + y0, x0 + y1, x1 + y1, iz0, corner);
+        tag = x0 + y0 + iz0;
+    }
+    return trilinear(corner, rx - i.flx, ry - i.fly, rz - i.flz);
+}
+
 template <bool CACHE, bool PER = false>
 __device__ __forceinline__ d3 grid_field_t(const DevGrid &g, d3 pos, Cand *cc) {
     if (!PER && g.interp != CRP_INTERPOLATION_TRILINEAR) {  // tricubic, nearest (Grid.h:328-331)
@@ -134,8 +172,6 @@ __device__ __forceinline__ d3 grid_field_t(const DevGrid &g, d3 pos, Cand *cc) {
         fY0 = ry - floor(ry);
         fZ0 = rz - floor(rz);
     }
-    const float fx1 = (float)(1 - fX0), fy1 = (float)(1 - fY0), fz1 = (float)(1 - fZ0);
-    const float fx0 = (float)fX0, fy0 = (float)fY0, fz0 = (float)fZ0;
     // cell indices: 32-bit for FS_GRID_PERIODIC grids (fewer than 2^31 cells)
     using Index = typename std::conditional<PER, unsigned, size_t>::type;
     const Index sy = (Index)g.nz, sx = (Index)g.ny * (Index)g.nz;
@@ -162,17 +198,7 @@ __device__ __forceinline__ d3 grid_field_t(const DevGrid &g, d3 pos, Cand *cc) {
         }
         if (CACHE) { cc->cell0 = k0; cc->cell7 = k7; cc->tag = (unsigned)(b00 + iz0); }
     }
-    const float wx[8] = {fx1, fx0, fx1, fx1, fx0, fx1, fx0, fx0};
-    const float wy[8] = {fy1, fy1, fy0, fy1, fy1, fy0, fy0, fy0};
-    const float wz[8] = {fz1, fz1, fz1, fz0, fz0, fz0, fz1, fz0};
-    float bx = 0.f, by = 0.f, bz = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        bx += c[k][0] * wx[k] * wy[k] * wz[k];
-        by += c[k][1] * wx[k] * wy[k] * wz[k];
-        bz += c[k][2] * wx[k] * wy[k] * wz[k];
-    }
-    return mk(bx, by, bz);
+    return trilinear(CACHE ? cc->corner : lc, fX0, fY0, fZ0);
 }
 
 __device__ d3 grid_field(const DevGrid &g, d3 pos) { return grid_field_t<false>(g, pos, nullptr); }
@@ -409,6 +435,97 @@ struct BP {
         set_current_step(c, step);
         c.next = newStep;
         return true;
+    }
+};
+
+// ------------------------------------------- the same push without divisions
+// IEEE divisions and square roots make half of the push's instructions (eighteen
+// divisions and two square roots of 652).  Every one of them divides by
+// something known beforehand (the grid spacing, the candidate's mass, c), shared
+// by three components (1 + t^2) or within rounding of 1 (the norms), and the
+// same correctly rounded quotients follow from a correctly rounded reciprocal
+// by fused remainders:
+//
+// a / b, rounded to nearest, for rb = 1 / b rounded to nearest (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990): the first correction leaves a quotient within one ulp, whose remainder
+// is exact, and the second rounds it correctly.  a and a / b nonzero and far
+// from the ends of the exponent range.
+__device__ __forceinline__ double quotient(double a, double b, double rb) {
+    double q = a * rb;
+    q = fma(fma(-q, b, a), rb, q);
+    return fma(fma(-q, b, a), rb, q);
+}
+__device__ __forceinline__ d3 quotient(d3 a, double b, double rb) {
+    return {quotient(a.x, b, rb), quotient(a.y, b, rb), quotient(a.z, b, rb)};
+}
+
+// u / |u| for n2 = u.u within 2^-27 of 1.  With n2 = 1 + e the square root is
+// 1 + e/2 - e^2/8, and e/2 is a multiple of half the spacing of doubles there:
+// the small last term only decides the ties, downwards, so rounding 1 + e/2 down
+// gives the correctly rounded root r.  In the same way 1/r = 1 - d + d^2 for
+// r = 1 + d is 2 - r with its ties rounded up.
+__device__ __forceinline__ d3 unit_near_1(d3 u, double n2) {
+    const double r = __fma_rd(0.5, n2, 0.5);
+    return quotient(u, r, __dsub_ru(2.0, r));
+}
+
+__device__ __forceinline__ int exponent_bits(double a) { return __double2hiint(a) & 0x7fffffff; }
+
+// The push of boris_body in the FP64 form: BP<FS_GRID_PERIODIC, 1>'s step, value
+// for value.
+struct BorisPush {
+    double q, mass, rmass;
+    unsigned tag;
+    float corner[8][3];
+    // The range in which every quotient of bp_dy and its remainders are normal
+    // numbers, for any nonzero float field value.
+    __device__ __forceinline__ static bool sane(const DevPlan &P, double q, double E) {
+        const double m = E / (kCLight * kCLight), step = P.modules[0].max_step;
+        return fabs(q) > 1e-60 && fabs(q) < 1e60 && m > 1e-60 && m < 1e60 && step > 1e-60 && step < 1e60;
+    }
+    __device__ __forceinline__ static double later(double time, double step) { return time + step / kCLight; }
+    __device__ __forceinline__ BorisPush(const DevPlan &P, double charge, double E) : q(charge) {
+        mass = E / (kCLight * kCLight);
+        rmass = 1.0 / mass;
+        tag = kNoCell;
+    }
+    __device__ __forceinline__ void step(const DevPlan &P, double &x, double &y, double &z, double &ux, double &uy,
+                                         double &uz) {
+        const DevGrid &g = P.fields[0].grid;
+        const double h = P.modules[0].max_step;
+        d3 X = mk(x, y, z), u = mk(ux, uy, uz);
+        X = add(X, divs(muls(u, h), 2.));
+        const d3 B = grid_periodic(g, X, tag, corner);
+        d3 t, s;
+        double D;
+        const float least = fminf(fabsf((float)B.x), fminf(fabsf((float)B.y), fabsf((float)B.z)));
+        bool plain = least > 0.f;
+        if (plain) {
+            t = quotient(muls(quotient(divs(muls(B, q), 2), mass, rmass), h), kCLight, 1.0 / kCLight);
+            D = 1 + dot(t, t);
+            plain = D < 1e150;
+            s = quotient(muls(t, 2), D, 1.0 / D);
+        }
+        if (!plain) {  // a component is zero or not finite
+            t = divs(muls(divs(divs(muls(B, q), 2), mass), h), kCLight);
+            D = 1 + dot(t, t);
+            s = divs(muls(t, 2), D);
+        }
+        const d3 vh = add(u, cross(u, t));
+        u = add(u, cross(vh, s));
+        X = add(X, divs(muls(u, h), 2.));
+        x = X.x; y = X.y; z = X.z;
+        const double n2 = u.x * u.x + u.y * u.y + u.z * u.z;
+        const int low = min(exponent_bits(u.x), min(exponent_bits(u.y), exponent_bits(u.z)));
+        if (fabs(n2 - 1) < 0x1p-27 && low > 0x07b00000) {  // every component above 2^-900
+            u = unit_near_1(u, n2);
+            u = unit_near_1(u, u.x * u.x + u.y * u.y + u.z * u.z);
+        } else {
+            u = unit(u);
+            u = divs(u, norm(u));
+        }
+        ux = u.x; uy = u.y; uz = u.z;
     }
 };
 
@@ -682,6 +799,19 @@ void for_signature(int fs, int shape, F f) {
         if (shape == CS_PMO) f(s, pmo);
         else f(s, any);
     }
+}
+
+// The boris_body kernel, 4 resident blocks of 128 threads per SM: bound by the
+// latency of dependent FP64 operations, which 116 registers hold without spills
+// (200 001 candidates x 1000 steps over 256^3 cells: 6.85 ms for the chain kernel
+// with its divisions, here 4.20 ms at 4 blocks, 4.31 at 5, 4.58 at 6; 20 011
+// candidates x 1500 steps over 64^3: 3.54 ms, then 1.49, 1.55 and 1.98 ms).
+constexpr int kBorisMinBlocks = 4;
+template <class Push>
+__global__ void __launch_bounds__(128, kBorisMinBlocks)
+fp64_boris_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, int lanes, int max_steps, uint64_t step_cap,
+                   DevCounters *cnt, DevRecords rec, const uint32_t *perm, uint32_t *perm_out) {
+    boris_body<Push, BPFixed<FS_GRID_PERIODIC>>(P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
 }
 
 template <template <int> class Prop>

@@ -1127,6 +1127,27 @@ struct BP {
     }
 };
 
+// The push of boris_body in the mixed form: BP<FS_GRID_PERIODIC, 1>'s step.
+struct BorisPush {
+    float kt;
+    unsigned tag;
+    float corner[8][3];
+    __device__ __forceinline__ static bool sane(const DevPlan &, double q, double) { return q != 0; }
+    __device__ __forceinline__ static double later(double time, double step) { return fma(step, kInvCLight, time); }
+    __device__ __forceinline__ BorisPush(const DevPlan &P, double q, double E) {
+        kt = boris_kq(q, E) * (float)P.modules[0].max_step;
+        tag = kNoCell;
+    }
+    __device__ __forceinline__ void step(const DevPlan &P, double &x, double &y, double &z, double &ux, double &uy,
+                                         double &uz) {
+        const double hh = 0.5 * P.modules[0].max_step;
+        x = fma(ux, hh, x); y = fma(uy, hh, y); z = fma(uz, hh, z);
+        const CellFrac f = grid_cell_load(P.fields[0].grid, x, y, z, tag, corner);
+        bp_rotate_drift(x, y, z, ux, uy, uz, grid_cell_interp(f, corner), kt, hh);
+        renorm(ux, uy, uz);
+    }
+};
+
 // --------------------------------------------------------------- Cash-Karp
 __constant__ float ck_af[36] = {
     0.f, 0.f, 0.f, 0.f, 0.f, 0.f,
@@ -1526,6 +1547,19 @@ void for_signature(int fs, int shape, F f) {
         if (shape == CS_PMO) f(s, pmo);
         else f(s, any);
     }
+}
+
+// The boris_body kernel, 7 resident blocks of 128 threads per SM: the loop's state
+// fits 72 registers without spills, and the loop waits for its corner gathers,
+// so more warps pay until 8 blocks spill (10^6 candidates x 5000 steps over 256^3
+// cells: 54.0 ms for the chain kernel at 6 blocks, here 48.1 ms at 6, 45.8 at 7,
+// 45.3 at 8; 20 011 candidates x 1000 steps: 0.80, 0.80 and 0.85 ms).
+constexpr int kBorisMinBlocks = 7;
+template <class Push>
+__global__ void __launch_bounds__(128, kBorisMinBlocks)
+mixed_boris_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, int lanes, int max_steps, uint64_t step_cap,
+                   DevCounters *cnt, DevRecords rec, const uint32_t *perm, uint32_t *perm_out) {
+    boris_body<Push, BPFixed<FS_GRID_PERIODIC>>(P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
 }
 
 template <template <int> class Prop>

@@ -12,6 +12,12 @@ cudaError_t launch_mixed_bp_chunk(const DevPlan &P, const DevState &s, uint64_t 
     if (n == 0) return cudaSuccess;
     const DevModule &pm = P.modules[P.prop_index];
     const bool fixed = pm.min_step == pm.max_step;
+    if (fixed && fs == FS_GRID_PERIODIC && P.shape == CS_PM) {
+        const uint64_t slots = (uint64_t)(block / 32) * (uint64_t)lanes;
+        mixed_boris_kernel<BorisPush><<<(unsigned)((n + slots - 1) / slots), block, 0, st>>>(
+            P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
+        return cudaGetLastError();
+    }
     return fixed ? launch_prop<BPFixed>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, lanes, st)
                  : launch_prop<BPAdaptive>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, lanes, st);
 }
