@@ -251,25 +251,28 @@ crp_status build_grid(crp_plan *p, const crp_grid3f_desc &g, int comps, DevGrid 
         return fail(CRP_ERR_CAPACITY, "%s: a dimension beyond 2^20 cells", name);
     if (g.interpolation < CRP_INTERPOLATION_TRILINEAR || g.interpolation > CRP_INTERPOLATION_NEAREST_NEIGHBOUR)
         return fail(CRP_ERR_INVALID_ARGUMENT, "%s: interpolation type not understood", name);
-    size_t cells = (size_t)g.nx * g.ny * g.nz;
-    crp_status st = upload(p, g.values, cells * comps, &dg.values);
-    if (st) return st;
+    const size_t cells = (size_t)g.nx * g.ny * g.nz;
     dg.pairs = nullptr;
-    if (comps == 3 && cells <= kPairCells) {
-        void *d = nullptr;
-        const cudaError_t e = cudaMalloc(&d, cells * 32);
-        if (e == cudaSuccess) {
-            p->owned.push_back(d);
-            pair_records_kernel<<<(unsigned)((cells + 255) / 256), 256>>>(dg.values, (unsigned)g.nz, (unsigned)cells,
-                                                                          static_cast<float4 *>(d));
-            CUDA_TRY(cudaGetLastError());
-            CUDA_TRY(cudaStreamSynchronize(0));  // runs may use any stream
-            dg.pairs = static_cast<const float *>(d);
-        } else if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();  // too large beside the grid: the packed values are read
-        } else {
-            return cuda_fail(e, "cudaMalloc(pair records)");
-        }
+    // records and values in one allocation
+    void *d = nullptr;
+    const size_t records = comps == 3 && cells <= kPairCells ? cells * 32 : 0;
+    cudaError_t e = records ? cudaMalloc(&d, records + cells * 12) : cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) {
+        p->owned.push_back(d);
+        float4 *pairs = static_cast<float4 *>(d);
+        float *values = static_cast<float *>(d) + records / sizeof(float);
+        CUDA_TRY(cudaMemcpy(values, g.values, cells * 12, cudaMemcpyHostToDevice));
+        pair_records_kernel<<<(unsigned)((cells + 255) / 256), 256>>>(values, (unsigned)g.nz, (unsigned)cells, pairs);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaStreamSynchronize(0));  // runs may use any stream
+        dg.values = values;
+        dg.pairs = reinterpret_cast<const float *>(pairs);
+    } else if (e == cudaErrorMemoryAllocation) {  // no records wanted, or no room for them: the packed values are read
+        if (records) cudaGetLastError();
+        const crp_status st = upload(p, g.values, cells * comps, &dg.values);
+        if (st) return st;
+    } else {
+        return cuda_fail(e, "cudaMalloc(Grid3f)");
     }
     dg.nx = (int)g.nx; dg.ny = (int)g.ny; dg.nz = (int)g.nz;
     dg.reflective = g.reflective;
