@@ -480,6 +480,56 @@ __device__ __forceinline__ void append_active(DevCounters *cnt, uint32_t *list, 
     if (still && list) list[base + __popc(mask & ((1u << lane) - 1u))] = index;
 }
 
+// advance() for kernels whose field is evaluated by the block: every thread
+// makes every pass and takes part in its field evaluations, those without an
+// open step with the state they have.
+template <class Prop, int CS>
+__device__ __forceinline__ int advance_block(const DevPlan &P, Cand &c, const DevRecords &rec, StepCount &sc,
+                                             int kmax) {
+    const int pi = CS == CS_GENERIC ? P.prop_index : 0;
+    const DevModule &pm = P.modules[pi];
+    typename Prop::Try t{};
+    bool open = false;
+    int k = 0;
+    while (__syncthreads_or(open || (c.active && k < kmax))) {
+        bool done = false;
+        if (!open && c.active && k < kmax) {
+            if (CS == CS_GENERIC) chain_part(P, c, rec, 0, pi);
+            open = Prop::begin(P, pm, c, t);
+            done = !open;
+        }
+        if (Prop::attempt(P, pm, c, t, sc, open)) {
+            done = true;
+            open = false;
+        }
+        if (done) {
+            if (CS == CS_GENERIC) {
+                chain_part(P, c, rec, pi + 1, P.n_modules);
+            } else {
+                max_trajectory_length(P.modules[1], c, rec, 1);
+                if (CS == CS_PMO) observer(P, P.modules[2], c, rec, 2);
+            }
+            if (Prop::kReadsStepCount) c.steps++;
+            k++;
+        }
+    }
+    if (!Prop::kReadsStepCount) c.steps += (uint64_t)k;
+    return k;
+}
+
+// A candidate of zeros for the threads of a block that hold none.
+__device__ __forceinline__ void no_cand(Cand &c) {
+    c.x = c.y = c.z = c.dx = c.dy = c.dz = c.px = c.py = c.pz = 0.;
+    c.E = c.q = 1.;
+    c.len = c.time = c.cur = c.next = c.maxlen = 0.;
+    c.index = c.steps = 0;
+    c.flags = 0;
+    c.id = 0;
+    c.active = false;
+    c.cell0 = c.cell7 = -1;
+    c.tag = kNoCell;
+}
+
 // The candidate slot of this thread: each warp takes `lanes` consecutive
 // slots (32: one per lane).  Small runs take fewer than 32 (lanes_per_warp,
 // engine_internal.h).
@@ -528,6 +578,37 @@ __device__ __forceinline__ void chunk_body(const DevPlan &P, const DevState &s, 
         store_cand(s, c);
     }
     flush_counters(cnt, steps, sc);
+    append_active(cnt, perm_out, still, (uint32_t)i);
+}
+
+// chunk_body for blocks that evaluate the field together: the first
+// 32 P.block_warps threads of each block hold a candidate.
+template <class Prop, int CS>
+__device__ __forceinline__ void chunk_block_body(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
+                                                 uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
+                                                 const uint32_t *perm_in, uint32_t *perm_out) {
+    const unsigned slots = 32u * (unsigned)P.block_warps;
+    const uint64_t t = threadIdx.x < slots ? (uint64_t)blockIdx.x * slots + threadIdx.x : n;
+    StepCount sc;
+    Cand c;
+    no_cand(c);
+    int kmax = 0;
+    bool loaded = false, still = false;
+    uint64_t i = 0;
+    if (t < n) {
+        i = perm_in ? perm_in[t] : t;
+        if (s.active[i]) {
+            load_cand(s, i, c);
+            kmax = launch_steps(c, max_steps, step_cap);
+            loaded = true;
+        }
+    }
+    const int k = advance_block<Prop, CS>(P, c, rec, sc, kmax);
+    if (loaded) {
+        still = c.active && (step_cap == 0 || c.steps < step_cap);
+        store_cand(s, c);
+    }
+    flush_counters(cnt, (unsigned long long)k, sc);
     append_active(cnt, perm_out, still, (uint32_t)i);
 }
 

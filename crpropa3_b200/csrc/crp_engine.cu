@@ -323,7 +323,7 @@ crp_status build_component(crp_plan *p, const crp_field_component &f, DevCompone
         std::vector<double> m9((size_t)n * 9);
         // mixed form, per pair of modes (a, b): {kx_a, ky_a, kz_a, kx_b, ky_b, kz_b} as doubles
         // (k kappa / 2 pi times 2^32: the phase in turns as 32-bit fixed point, exact scaling),
-        // then {beta_a, beta_b} as unsigned 32-bit fixed-point turns and {A xi_a, A xi_b} as
+        // then {beta_a, beta_b} as unsigned 32-bit fixed-point turns plus kWaveBias and {A xi_a, A xi_b} as
         // floats: 48 + 8 + 24 = 80 bytes, five 16-byte loads
         const int npairs = (n + 1) / 2;
         std::vector<float4> pairs((size_t)npairs * 5);
@@ -351,7 +351,7 @@ crp_status build_component(crp_plan *p, const crp_field_component &f, DevCompone
             // beta / 2 pi in [0, 1) turns, as 32-bit fixed point
             double bt = w.beta[i] * kInv2Pi;
             bt -= std::floor(bt);
-            bu[h] = (uint32_t)(int64_t)std::llround(bt * kTurnScale);
+            bu[h] = (uint32_t)(int64_t)std::llround(bt * kTurnScale) + kWaveBias;
         }
         crp_status st = upload(p, m9.data(), m9.size(), &d.pw.modes);
         if (st) return st;

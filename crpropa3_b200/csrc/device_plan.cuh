@@ -31,6 +31,10 @@ struct DevGrid {
     int pad_;
 };
 
+// What cos_turns (mixed_device.cuh) adds to a mode's fixed-point phase: half a
+// turn and the rounding of the 23 bits it keeps.  The mode table's beta has it.
+constexpr uint32_t kWaveBias = 0x80000000u + 256u;
+
 struct DevPlaneWave {
     const double *modes;   // FP64 form: per mode {xi x y z, kappa x y z, k, beta, Ak} (9 doubles)
     const float4 *pairs;   // mixed form: the modes in pairs, 80 B = 5 x 16 B per pair (step_mixed.cu)
@@ -173,6 +177,7 @@ struct DevPlan {
     int n_modules;
     int prop_index;  // position of the propagation module in the chain
     int shape;       // ChainShape (chain.cuh) the module sequence matches
+    int block_warps; // FS_PLANE_WAVE_BLOCK: warps of a block that hold candidates (set per launch)
     uint64_t seed;
     DevComponent fields[kMaxFields];
     const DevComponent *dev_fields;  // device copy of the n_fields components (field_sum)

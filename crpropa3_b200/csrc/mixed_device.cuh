@@ -232,21 +232,21 @@ struct PwTab {
 };
 
 // cos(2 pi (p + beta)) for a phase p in turns given as p * 2^32 (the table's
-// scale) and beta in 32-bit fixed-point turns.  FAST (|p * 2^32| < 2^50):
-// adding 1.5 * 2^52 rounds p * 2^32 to an integer whose low 32 bits are the
-// fraction of a turn in fixed point; beta is added there (mod 2^32), and the
-// sum's top 23 bits, shifted by half a turn, become a float in [-1/2, 1/2)
-// through the exponent bits of 1.0 (no conversion instruction, 2^-23-turn
-// steps, rounded).  Otherwise the FP64 fraction of p + beta rounded to FP32.
+// scale) and beta in 32-bit fixed-point turns plus kWaveBias.  FAST
+// (|p * 2^32| < 2^50): adding 1.5 * 2^52 rounds p * 2^32 to an integer whose low
+// 32 bits are the fraction of a turn in fixed point; beta is added there (mod
+// 2^32), with half a turn and half a unit of the 23 bits kept, and the sum's top
+// 23 bits become a float in [-1/2, 1/2) through the exponent bits of 1.0 (one
+// addition and one funnel shift, no conversion; 2^-23-turn steps, rounded).  Otherwise the FP64 fraction of p + beta rounded to FP32.
 template <bool FAST>
 __device__ __forceinline__ float cos_turns(double ps, unsigned beta) {
     const float twopi = 6.28318530717958647692f;
     if (FAST) {
-        const unsigned lo = (unsigned)__double2loint(ps + 6755399441055744.0) + beta;
-        const float f = __int_as_float(0x3f800000u | (((lo + 256u) ^ 0x80000000u) >> 9)) - 1.5f;
+        const unsigned v = (unsigned)__double2loint(ps + 6755399441055744.0) + beta;
+        const float f = __int_as_float(__funnelshift_r(v, 0x7fu, 9)) - 1.5f;  // 0x3f800000 | v >> 9
         return __cosf(twopi * f);
     }
-    const double p = (ps + (double)beta) * 2.3283064365386962890625e-10;  // 2^-32, exact
+    const double p = (ps + (double)(beta - kWaveBias)) * 2.3283064365386962890625e-10;  // 2^-32, exact
     return __cosf(twopi * (float)(p - rint(p)));
 }
 
@@ -315,6 +315,96 @@ __device__ __forceinline__ f3 plane_wave_field(const DevPlaneWave &w, double x, 
                                                const PwTab *sh = nullptr) {
     if (sh) return pw_sum<true>(sh->pairs, sh->npairs, sh->fast_limit, x, y, z);
     return pw_sum<false>(w.pairs, w.npairs, w.fast_limit, x, y, z);
+}
+
+constexpr int kBatchThreads = 128;  // 4 warps: one per mode group
+
+// Group sums of warp `g` for the positions lane + 32 j (j < NP) of the
+// block's query list; positions at or past `total` are computed on the first
+// query and not written.
+template <int NP, bool ALL_FAST>
+__device__ __forceinline__ void pw_batch_group(const float4 *tab, int q0, int q1, const double *qpos, int total,
+                                               double lim, float *part, int g) {
+    const int lane = threadIdx.x & 31;
+    double x[NP], y[NP], z[NP];
+    bool fast[NP];
+    float acc[NP][6];
+#pragma unroll
+    for (int j = 0; j < NP; j++) {
+        const int p = lane + 32 * j < total ? lane + 32 * j : 0;
+        x[j] = qpos[p]; y[j] = qpos[kBatchThreads + p]; z[j] = qpos[2 * kBatchThreads + p];
+        fast[j] = fmax(fabs(x[j]), fmax(fabs(y[j]), fabs(z[j]))) < lim;
+#pragma unroll
+        for (int a = 0; a < 6; a++) acc[j][a] = 0.f;
+    }
+#pragma unroll 2
+    for (int q = q0; q < q1; q++) {
+        const double2 *kd = reinterpret_cast<const double2 *>(tab + 5 * q);
+        const double2 k0 = kd[0], k1 = kd[1], k2 = kd[2];
+        const float4 u = tab[5 * q + 3], v = tab[5 * q + 4];
+#pragma unroll
+        for (int j = 0; j < NP; j++) {
+            if (ALL_FAST || fast[j]) pw_pair_add<true>(k0, k1, k2, u, v, x[j], y[j], z[j], acc[j]);
+            else pw_pair_add<false>(k0, k1, k2, u, v, x[j], y[j], z[j], acc[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NP; j++) {
+        const int p = lane + 32 * j;
+        if (p < total) {
+            float *o = part + (size_t)g * 3 * kBatchThreads;
+            o[p] = acc[j][0] + acc[j][3];
+            o[kBatchThreads + p] = acc[j][1] + acc[j][4];
+            o[2 * kBatchThreads + p] = acc[j][2] + acc[j][5];
+        }
+    }
+}
+
+template <bool ALL_FAST>
+__device__ __forceinline__ void pw_batch(const float4 *tab, int npairs, const double *qpos, int total, double lim,
+                                         float *part) {
+    const int g = threadIdx.x >> 5;
+    const int q0 = pw_group_begin(npairs, g), q1 = g + 1 < kPwGroups ? pw_group_begin(npairs, g + 1) : npairs;
+    const int np = (total + 31) >> 5;  // positions per lane, uniform over the block
+    if (np == 1) pw_batch_group<1, ALL_FAST>(tab, q0, q1, qpos, total, lim, part, g);
+    else if (np == 2) pw_batch_group<2, ALL_FAST>(tab, q0, q1, qpos, total, lim, part, g);
+    else if (np == 3) pw_batch_group<3, ALL_FAST>(tab, q0, q1, qpos, total, lim, part, g);
+    else pw_batch_group<4, ALL_FAST>(tab, q0, q1, qpos, total, lim, part, g);
+}
+
+// The block's copy of the mode table.
+inline size_t wave_table_bytes(const DevPlaneWave &w) { return (size_t)w.npairs * 80; }
+__device__ __forceinline__ void stage_wave_table(const DevPlaneWave &w, unsigned char *to) {
+    float4 *t4 = reinterpret_cast<float4 *>(to);
+    for (int q = threadIdx.x; q < 5 * w.npairs; q += blockDim.x) t4[q] = __ldg(w.pairs + q);
+}
+
+// PlaneWaveTurbulence evaluated by a block for its candidates (FS_PLANE_WAVE_BLOCK
+// kernels; every thread of the block calls it).  A thread's mode sum is a chain
+// of dependent operations hundreds of modes long, and a run of 10^4 candidates
+// has one warp per scheduler to hide it with; here the block's first 32 wp
+// threads hold the candidates, their positions go through shared memory, and warp
+// g sums mode group g for all of them, wp positions per lane and table read.
+// The sums are those of pw_sum_t, operation for operation.  20 000 candidates x
+// 200 steps x 200 modes: 2.06 ms thread by thread, 1.01 ms here.
+__device__ __forceinline__ f3 plane_wave_block(const DevPlaneWave &w, double x, double y, double z, int wp) {
+    __shared__ double qpos[3 * kBatchThreads];
+    __shared__ float part[kPwGroups * 3 * kBatchThreads];
+    extern __shared__ __align__(16) unsigned char pw_table[];
+    const int t = threadIdx.x;
+    qpos[t] = x; qpos[kBatchThreads + t] = y; qpos[2 * kBatchThreads + t] = z;
+    const bool fast = t >= 32 * wp || fmax(fabs(x), fmax(fabs(y), fabs(z))) < w.fast_limit;
+    const float4 *tab = reinterpret_cast<const float4 *>(pw_table);
+    if (__syncthreads_and(fast)) pw_batch<true>(tab, w.npairs, qpos, 32 * wp, w.fast_limit, part);
+    else pw_batch<false>(tab, w.npairs, qpos, 32 * wp, w.fast_limit, part);
+    __syncthreads();
+    f3 g[kPwGroups];
+#pragma unroll
+    for (int i = 0; i < kPwGroups; i++) {
+        const float *o = part + i * 3 * kBatchThreads + t;
+        g[i] = f3mk(o[0], o[kBatchThreads], o[2 * kBatchThreads]);
+    }
+    return pw_combine(g[0], g[1], g[2], g[3]);
 }
 
 // ---------------------------------------------------------------- JF12Field
@@ -1003,6 +1093,7 @@ __device__ __forceinline__ f3 field_at(const DevPlan &P, double x, double y, dou
     if (FS == FS_GRID) return grid_field_t<true, false, FUSED>(P.fields[0].grid, x, y, z, cc);
     if (FS == FS_GRID_PERIODIC) return grid_field_t<true, true>(P.fields[0].grid, x, y, z, cc);
     if (FS == FS_PLANE_WAVE) return plane_wave_field(P.fields[0].pw, x, y, z, sh);
+    if (FS == FS_PLANE_WAVE_BLOCK) return plane_wave_block(P.fields[0].pw, x, y, z, P.block_warps);
     return field_sum(P.dev_fields, P.n_fields, x, y, z, sh);
 }
 
@@ -1068,6 +1159,7 @@ __device__ __forceinline__ void bp_dy(const DevPlan &P, double &x, double &y, do
 template <int FS, int MODE = 0>
 struct BP {
     static constexpr bool kReadsStepCount = false;
+    static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
     static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
     struct Try {
         double step;
@@ -1084,14 +1176,16 @@ struct BP {
         t.guard = 0;
         return true;
     }
-    // One try; true when the step is done.
+    // One try; true when the step is done.  Threads that only take part in the
+    // field evaluations pass on = false.
     __device__ __forceinline__ static bool attempt(const DevPlan &P, const DevModule &m, Cand &c, Try &t,
-                                                   StepCount &sc) {
+                                                   StepCount &sc, bool on = true) {
         double step = t.step, newStep = step;
         const float kq = boris_kq(c.q, c.E);
         double xo = c.x, yo = c.y, zo = c.z, uxo = c.dx, uyo = c.dy, uzo = c.dz;
         if (MODE == 1) {
             bp_dy<FS, true>(P, xo, yo, zo, uxo, uyo, uzo, step, kq * (float)step, &c);
+            if (!on) return false;
             sc.tries++; sc.evals++;
         } else {
             // the full step, then two half steps: one loop body for the three
@@ -1108,6 +1202,7 @@ struct BP {
                     kt = 0.5f * kts;
                 }
             }
+            if (!on) return false;
             sc.tries++; sc.evals += 3;
             double ex = xo - x, ey = yo - y, ez = zo - z;
             double S = sqrt(norm2(ex, ey, ez)) / (step * 0.75);
@@ -1206,6 +1301,7 @@ __device__ __forceinline__ double ck_try(const DevPlan &P, Cand &c, double h, fl
 template <int FS, int MODE = 0>
 struct CK {
     static constexpr bool kReadsStepCount = false;
+    static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
     static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
     struct Try {
         double step;
@@ -1222,11 +1318,12 @@ struct CK {
         return true;
     }
     __device__ __forceinline__ static bool attempt(const DevPlan &P, const DevModule &m, Cand &c, Try &t,
-                                                   StepCount &sc) {
+                                                   StepCount &sc, bool on = true) {
         double step = t.step, newStep = step;
         const float qc2E = __fdividef((float)(c.q * (kCLight * kCLight)), (float)c.E);
         double xo, yo, zo, dux, duy, duz;
         const double err = ck_try<FS>(P, c, step * kInvCLight, qc2E, xo, yo, zo, dux, duy, duz);
+        if (!on) return false;
         sc.tries++; sc.evals += 6;
         if (MODE != 1) {
             const double r = err / m.tolerance;
@@ -1475,6 +1572,7 @@ __device__ __forceinline__ bool sde_co_consume(const DevPlan &P, const DevModule
 template <int FS>
 struct SDE {
     static constexpr bool kReadsStepCount = true;  // the Philox counter
+    static constexpr bool kBlockField = false;
     static constexpr bool kRetries = false;
     struct Try {};
     __device__ __forceinline__ static bool begin(const DevPlan &, const DevModule &, Cand &, Try &) { return true; }
@@ -1562,11 +1660,45 @@ mixed_boris_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, in
     boris_body<Push, BPFixed<FS_GRID_PERIODIC>>(P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
 }
 
+// Kernels of FS_PLANE_WAVE_BLOCK: the mode table staged in dynamic shared memory.
+template <template <int> class Prop, int CS>
+__global__ void __launch_bounds__(kBatchThreads, 4)
+mixed_wave_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, int max_steps, uint64_t step_cap,
+                  DevCounters *cnt, DevRecords rec, const uint32_t *perm, uint32_t *perm_out) {
+    extern __shared__ __align__(16) unsigned char pw_table[];
+    stage_wave_table(P.fields[0].pw, pw_table);
+    __syncthreads();
+    chunk_block_body<Prop<FS_PLANE_WAVE_BLOCK>, CS>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out);
+}
+
+template <template <int> class Prop>
+cudaError_t launch_waves(DevPlan P, const DevState &s, uint64_t n, int max_steps, uint64_t step_cap, DevCounters *cnt,
+                         const DevRecords &rec, const uint32_t *perm, uint32_t *perm_out, int warps, cudaStream_t st) {
+    P.block_warps = warps;
+    const size_t smem = wave_table_bytes(P.fields[0].pw);
+    const unsigned grid = (unsigned)((n + 32 * warps - 1) / (32 * warps));
+    auto launch = [&](auto c) {
+        auto kernel = mixed_wave_kernel<Prop, decltype(c)::value>;
+        // beside the kernel's own shared memory
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kernel<<<grid, kBatchThreads, smem, st>>>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out);
+        return cudaGetLastError();
+    };
+    if (P.shape == CS_PM) return launch(std::integral_constant<int, CS_PM>());
+    if (P.shape == CS_PMO) return launch(std::integral_constant<int, CS_PMO>());
+    return launch(std::integral_constant<int, CS_GENERIC>());
+}
+
 template <template <int> class Prop>
 cudaError_t launch_prop(const DevPlan &P, const DevState &s, uint64_t n, int max_steps,
                         uint64_t step_cap, DevCounters *cnt, const DevRecords &rec,
                         const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
                         cudaStream_t st) {
+    if constexpr (Prop<FS_PLANE_WAVE>::kBlockField) {
+        const int warps = fs == FS_PLANE_WAVE ? wave_block_warps(n, P.fields[0].pw.n, false) : 0;
+        if (warps) return launch_waves<Prop>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, warps, st);
+    }
     const uint64_t slots = (uint64_t)(block / 32) * (uint64_t)lanes;
     const unsigned grid = (unsigned)((n + slots - 1) / slots);
     for_signature(fs, P.shape, [&](auto f, auto c) {

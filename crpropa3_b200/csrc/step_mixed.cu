@@ -114,61 +114,6 @@ __global__ void __launch_bounds__(128, CRP_SDE_COOP_MIN_BLOCKS) mixed_sde_coop_k
 #ifndef CRP_SDE_BATCH_MIN_BLOCKS
 #define CRP_SDE_BATCH_MIN_BLOCKS 2
 #endif
-constexpr int kBatchThreads = 128;  // 4 warps: one per mode group
-
-// Group sums of warp `g` for the positions lane + 32 j (j < NP) of the
-// block's query list; positions at or past `total` are computed on the first
-// query and not written.
-template <int NP, bool ALL_FAST>
-__device__ __forceinline__ void pw_batch_group(const float4 *tab, int q0, int q1, const double *qpos, int total,
-                                               double lim, float *part, int g) {
-    const int lane = threadIdx.x & 31;
-    double x[NP], y[NP], z[NP];
-    bool fast[NP];
-    float acc[NP][6];
-#pragma unroll
-    for (int j = 0; j < NP; j++) {
-        const int p = lane + 32 * j < total ? lane + 32 * j : 0;
-        x[j] = qpos[p]; y[j] = qpos[kBatchThreads + p]; z[j] = qpos[2 * kBatchThreads + p];
-        fast[j] = fmax(fabs(x[j]), fmax(fabs(y[j]), fabs(z[j]))) < lim;
-#pragma unroll
-        for (int a = 0; a < 6; a++) acc[j][a] = 0.f;
-    }
-#pragma unroll 2
-    for (int q = q0; q < q1; q++) {
-        const double2 *kd = reinterpret_cast<const double2 *>(tab + 5 * q);
-        const double2 k0 = kd[0], k1 = kd[1], k2 = kd[2];
-        const float4 u = tab[5 * q + 3], v = tab[5 * q + 4];
-#pragma unroll
-        for (int j = 0; j < NP; j++) {
-            if (ALL_FAST || fast[j]) pw_pair_add<true>(k0, k1, k2, u, v, x[j], y[j], z[j], acc[j]);
-            else pw_pair_add<false>(k0, k1, k2, u, v, x[j], y[j], z[j], acc[j]);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NP; j++) {
-        const int p = lane + 32 * j;
-        if (p < total) {
-            float *o = part + (size_t)g * 3 * kBatchThreads;
-            o[p] = acc[j][0] + acc[j][3];
-            o[kBatchThreads + p] = acc[j][1] + acc[j][4];
-            o[2 * kBatchThreads + p] = acc[j][2] + acc[j][5];
-        }
-    }
-}
-
-template <bool ALL_FAST>
-__device__ __forceinline__ void pw_batch(const float4 *tab, int npairs, const double *qpos, int total, double lim,
-                                         float *part) {
-    const int g = threadIdx.x >> 5;
-    const int q0 = pw_group_begin(npairs, g), q1 = g + 1 < kPwGroups ? pw_group_begin(npairs, g + 1) : npairs;
-    const int np = (total + 31) >> 5;  // positions per lane, uniform over the block
-    if (np == 1) pw_batch_group<1, ALL_FAST>(tab, q0, q1, qpos, total, lim, part, g);
-    else if (np == 2) pw_batch_group<2, ALL_FAST>(tab, q0, q1, qpos, total, lim, part, g);
-    else if (np == 3) pw_batch_group<3, ALL_FAST>(tab, q0, q1, qpos, total, lim, part, g);
-    else pw_batch_group<4, ALL_FAST>(tab, q0, q1, qpos, total, lim, part, g);
-}
-
 template <int FS>
 __global__ void __launch_bounds__(kBatchThreads, CRP_SDE_BATCH_MIN_BLOCKS)
 mixed_sde_batch_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, int max_steps, uint64_t step_cap, DevCounters *cnt,
