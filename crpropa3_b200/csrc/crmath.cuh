@@ -131,10 +131,76 @@ CRP_HD dd dd_exp(dd t) {
     return r;
 }
 
+// x^y for normal x, |y| <= 1, to a relative error below 2^-63 and rounded, if that
+// error cannot change the rounding (true for all but 0.8 % of inputs).  The
+// same reductions as below, with the leading terms of each series in
+// double-double and their tails, at most 2^-12.5 of the sum, in double:
+//   log: s = (m-1)/(m+1), z = s^2 <= 0.0295: 2 s (1 + z/3 + z^2 P(z)); error of the
+//        tail 3 ulp of 2^-12.5 times |2 s| <= 0.35: below 2^-64.5;
+//   exp: v = u / 8, |v| <= 0.0434: v + v^2/2 + v^3 Q(v); error of the tail 3 ulp of
+//        2^-16: 2^-67.5, three doublings of the argument: below 2^-64.
+// A tenth of the full evaluation's operations.
+CRP_HD bool pow_quick(double x, double y, double &result) {
+    int k;
+    double m = frexp(x, &k);
+    if (m < 0.70710678118654752440) {
+        m *= 2.0;
+        k -= 1;
+    }
+    const double num = m - 1.0;
+    const dd den = dd_fast_two_sum(m > 1.0 ? m : 1.0, m > 1.0 ? 1.0 : m);
+    const double inv = 1.0 / den.hi;
+    const double q1 = num * inv;
+    const double q2 = fma(-q1, den.lo, fma(-q1, den.hi, num)) * inv;
+    const double zh = q1 * q1, zl = fma(q1, q1, -zh) + 2.0 * q1 * q2;
+    double P = 1.0 / 27.0;
+    P = fma(P, zh, 1.0 / 25.0); P = fma(P, zh, 1.0 / 23.0); P = fma(P, zh, 1.0 / 21.0);
+    P = fma(P, zh, 1.0 / 19.0); P = fma(P, zh, 1.0 / 17.0); P = fma(P, zh, 1.0 / 15.0);
+    P = fma(P, zh, 1.0 / 13.0); P = fma(P, zh, 1.0 / 11.0); P = fma(P, zh, 1.0 / 9.0);
+    P = fma(P, zh, 1.0 / 7.0); P = fma(P, zh, 1.0 / 5.0);
+    const double third = 1.0 / 3.0, third_lo = 1.0 / 54043195528445952.0;  // 1/3 - RN(1/3) = 2^-54 / 3
+    const double p = zh * third, pe = fma(zh, third, -p) + zh * third_lo + zl * third;
+    const dd B = dd_fast_two_sum(p, zh * zh * P);
+    const double Bl = B.lo + pe;
+    const double w = q1 * B.hi, we = fma(q1, B.hi, -w) + q1 * Bl + q2 * B.hi + q2;
+    const dd l = dd_fast_two_sum(q1, w);
+    const double a = k * CRP_LN2_HI, ae = fma((double)k, CRP_LN2_HI, -a) + k * CRP_LN2_LO;
+    const dd L = dd_two_sum(a, 2.0 * l.hi);
+    const double Ll = L.lo + (2.0 * (l.lo + we) + ae);
+    const double th = y * L.hi, tl = fma(y, L.hi, -th) + y * Ll;
+    if (!(fabs(th) < 699.0)) return false;
+    const double j = rint(th * (1.0 / CRP_LN2_HI));
+    const double b = j * CRP_LN2_HI;
+    const dd u = dd_fast_two_sum(th - b, (tl - fma(j, CRP_LN2_HI, -b)) - j * CRP_LN2_LO);
+    const double vh = 0.125 * u.hi, vl = 0.125 * u.lo;
+    const double ah = vh * vh, al = fma(vh, vh, -ah) + 2.0 * vh * vl;
+    double Q = 1.0 / 3628800.0;
+    Q = fma(Q, vh, 1.0 / 362880.0); Q = fma(Q, vh, 1.0 / 40320.0); Q = fma(Q, vh, 1.0 / 5040.0);
+    Q = fma(Q, vh, 1.0 / 720.0); Q = fma(Q, vh, 1.0 / 120.0); Q = fma(Q, vh, 1.0 / 24.0);
+    Q = fma(Q, vh, 1.0 / 6.0);
+    const dd e0 = dd_fast_two_sum(vh, 0.5 * ah);
+    const dd e1 = dd_fast_two_sum(e0.hi, vh * ah * Q);
+    double eh = e1.hi, el = e1.lo + e0.lo + vl + 0.5 * al;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {  // (1 + e)^2 - 1 = 2 e + e^2
+        const double sq = eh * eh, sl = fma(eh, eh, -sq) + 2.0 * eh * el;
+        const dd t = dd_fast_two_sum(2.0 * eh, sq);
+        eh = t.hi;
+        el = t.lo + 2.0 * el + sl;
+    }
+    const dd r = dd_fast_two_sum(1.0, eh);
+    const double lo = r.lo + el, eps = 4.336808689942018e-19;  // 2^-61 (r.hi in [0.7, 1.42])
+    const double below = r.hi + (lo - eps), above = r.hi + (lo + eps);
+    result = ldexp(below, (int)j);
+    return below == above;
+}
+
 CRP_HD double cr_pow(double x, double y) {
     if (!(x > 0.0) || !(x < INFINITY) || !(fabs(y) < INFINITY) || x < 2.2250738585072014e-308)
         return pow(x, y);
     if (y == 0.0 || x == 1.0) return 1.0;
+    double quick;
+    if (fabs(y) <= 1.0 && pow_quick(x, y, quick)) return quick;
     dd l = dd_log(x);
     dd t = dd_mul_d(l, y);
     if (!(fabs(t.hi) < 700.0)) return pow(x, y);

@@ -544,8 +544,14 @@ crp_status build_component(crp_plan *p, const crp_field_component &f, DevCompone
     return CRP_OK;
 }
 
+// The run counters, and the device copy of the field components beside them.
 crp_status ensure_counters(crp_plan *p) {
-    if (!p->d_cnt) CUDA_TRY(cudaMalloc(&p->d_cnt, sizeof(DevCounters)));
+    if (!p->d_cnt) {
+        CUDA_TRY(cudaMalloc(&p->d_cnt, sizeof(DevCounters) + sizeof(p->dev.fields)));
+        DevComponent *fields = reinterpret_cast<DevComponent *>(p->d_cnt + 1);
+        CUDA_TRY(cudaMemcpy(fields, p->dev.fields, sizeof(p->dev.fields), cudaMemcpyHostToDevice));
+        p->dev.dev_fields = fields;
+    }
     if (!p->h_cnt) CUDA_TRY(cudaMallocHost(&p->h_cnt, sizeof(DevCounters)));
     if (!p->ev0) CUDA_TRY(cudaEventCreate(&p->ev0));
     if (!p->ev1) CUDA_TRY(cudaEventCreate(&p->ev1));
@@ -651,11 +657,6 @@ crp_status crp_plan_create(const crp_plan_desc *desc, crp_plan **out) {
         d.shape = CS_PMO;
     for (int i = 0; i < desc->n_fields; i++) {
         crp_status st = build_component(p, desc->fields[i], d.fields[i]);
-        if (st) { delete p; return st; }
-    }
-    d.dev_fields = nullptr;
-    if (d.n_fields > 0) {
-        crp_status st = upload(p, d.fields, (size_t)d.n_fields, &d.dev_fields);
         if (st) { delete p; return st; }
     }
     int nfeat_total = 0;

@@ -66,6 +66,72 @@ __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b 
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
 __device__ __forceinline__ double clipd(double x, double lo, double hi) { return dmax(lo, dmin(x, hi)); }
 
+// ------------------------------------------------- quotients without divisions
+// IEEE divisions and square roots made half of the instructions of a Boris step
+// (eighteen divisions and two square roots of 652) and a third of a Cash-Karp
+// try's (36 divisions).  Every one of them divides by something known beforehand
+// (the grid spacing, the candidate's mass, c), shared by three components (1 +
+// t^2, the norms) or within rounding of 1 (a norm taken again), and the same
+// correctly rounded quotients follow from a correctly rounded reciprocal by fused
+// remainders:
+//
+// a / b, rounded to nearest, for rb = 1 / b rounded to nearest (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990): the first correction leaves a quotient within one ulp, whose remainder
+// is exact, and the second rounds it correctly.  a and a / b nonzero and far
+// from the ends of the exponent range.
+__device__ __forceinline__ double quotient(double a, double b, double rb) {
+    double q = a * rb;
+    q = fma(fma(-q, b, a), rb, q);
+    return fma(fma(-q, b, a), rb, q);
+}
+__device__ __forceinline__ d3 quotient(d3 a, double b, double rb) {
+    return {quotient(a.x, b, rb), quotient(a.y, b, rb), quotient(a.z, b, rb)};
+}
+
+// u / |u| for n2 = u.u within 2^-27 of 1.  With n2 = 1 + e the square root is
+// 1 + e/2 - e^2/8, and e/2 is a multiple of half the spacing of doubles there:
+// the small last term only decides the ties, downwards, so rounding 1 + e/2 down
+// gives the correctly rounded root r.  In the same way 1/r = 1 - d + d^2 for
+// r = 1 + d is 2 - r with its ties rounded up.
+__device__ __forceinline__ d3 unit_near_1(d3 u, double n2) {
+    const double r = __fma_rd(0.5, n2, 0.5);
+    return quotient(u, r, __dsub_ru(2.0, r));
+}
+
+__device__ __forceinline__ int exponent_bits(double a) { return __double2hiint(a) & 0x7fffffff; }
+
+// Every component above 2^-900, so that quotients by an ordinary number have
+// exact remainders.
+__device__ __forceinline__ bool ordinary(d3 u) {
+    return min(exponent_bits(u.x), min(exponent_bits(u.y), exponent_bits(u.z))) > 0x07b00000;
+}
+
+// unit(u), value for value.
+__device__ __forceinline__ d3 unit_fast(d3 u) {
+    const double r = norm(u);
+    if (ordinary(u) && r > 1e-100 && r < 1e100) return quotient(u, r, 1.0 / r);
+    return divs(u, r);
+}
+
+// ParticleState::setDirection after getUnitVector: u / |u| twice, value for value.
+__device__ __forceinline__ d3 unit_twice(d3 u) {
+    const double n2 = u.x * u.x + u.y * u.y + u.z * u.z;
+    if (ordinary(u) && n2 > 1e-100 && n2 < 1e100) {
+        if (fabs(n2 - 1) < 0x1p-27) {
+            u = unit_near_1(u, n2);
+        } else {
+            const double r = sqrt(n2);
+            u = quotient(u, r, 1.0 / r);
+        }
+        const double again = u.x * u.x + u.y * u.y + u.z * u.z;
+        if (ordinary(u) && fabs(again - 1) < 0x1p-27) return unit_near_1(u, again);
+        return divs(u, norm(u));
+    }
+    u = unit(u);
+    return divs(u, norm(u));
+}
+
 // i mod n in [0, n); positions inside the grid need no division.
 __device__ __forceinline__ int grid_wrap(int i, int n) {
     if ((unsigned)i < (unsigned)n) return i;
@@ -94,9 +160,6 @@ __device__ __forceinline__ d3 trilinear(const float (&c)[8][3], double fX0, doub
     }
     return mk(bx, by, bz);
 }
-
-// a / b rounded to nearest by a reciprocal, defined with the division-free push below.
-__device__ __forceinline__ double quotient(double a, double b, double rb);
 
 // The periodic power-of-two grid (PER below) with its own corner cache.  The
 // coordinates are quotients by the spacing (g.inv_s*: its correctly rounded
@@ -129,9 +192,8 @@ __device__ __forceinline__ d3 grid_field_t(const DevGrid &g, d3 pos, Cand *cc) {
         in &= (pos.z >= g.oz) && (pos.z <= g.ez);
         if (!in) return mk(0, 0, 0);
     }
-    double rx = (pos.x - g.gox) / g.sx;
-    double ry = (pos.y - g.goy) / g.sy;
-    double rz = (pos.z - g.goz) / g.sz;
+    const double rx = quotient(pos.x - g.gox, g.sx, g.inv_sx), ry = quotient(pos.y - g.goy, g.sy, g.inv_sy),
+                 rz = quotient(pos.z - g.goz, g.sz, g.inv_sz);
     int ix0, ix1, iy0, iy1, iz0, iz1;
     double fX0, fY0, fZ0;
     if (!PER && g.reflective) {  // reflectiveClamp (Grid.h:49)
@@ -405,15 +467,47 @@ __device__ __forceinline__ void set_current_step(Cand &c, double s) {  // Candid
 }
 
 // ---------------------------------------------------------------- Boris push
+// A candidate's factors of the rotation vector t = B q / 2 / m * step / c.
+// plain: the range in which every quotient of the push and its remainder is a
+// normal number for any nonzero float field value and steps of 1e-60 to 1e60 m.
+struct BorisFactors {
+    double q, mass, rmass;
+    bool plain;
+    __device__ __forceinline__ BorisFactors(double charge, double E) : q(charge) {
+        mass = E / (kCLight * kCLight);
+        rmass = 1.0 / mass;
+        plain = fabs(q) > 1e-60 && fabs(q) < 1e60 && mass > 1e-60 && mass < 1e60;
+    }
+};
+__device__ __forceinline__ bool plain_step(double step) { return step > 1e-60 && step < 1e60; }
+
+// PropagationBP::dY (PropagationBP.cpp:19) after the first half drift: the
+// rotation in the field B.  PLAIN: the factors and the step are known to be plain.
+template <bool PLAIN>
+__device__ __forceinline__ d3 boris_rotate(d3 u, d3 B, double step, const BorisFactors &f) {
+    d3 t, s;
+    double D;
+    const float least = fminf(fabsf((float)B.x), fminf(fabsf((float)B.y), fabsf((float)B.z)));
+    bool plain = least > 0.f && (PLAIN || (f.plain && plain_step(step)));
+    if (plain) {
+        t = quotient(muls(quotient(divs(muls(B, f.q), 2), f.mass, f.rmass), step), kCLight, 1.0 / kCLight);
+        D = 1 + dot(t, t);
+        plain = D < 1e150;
+        s = quotient(muls(t, 2), D, 1.0 / D);
+    }
+    if (!plain) {  // a component is zero or not finite
+        t = divs(muls(divs(divs(muls(B, f.q), 2), f.mass), step), kCLight);
+        D = 1 + dot(t, t);
+        s = divs(muls(t, 2), D);
+    }
+    const d3 vh = add(u, cross(u, t));
+    return add(u, cross(vh, s));
+}
+
 template <int FS>
-__device__ __forceinline__ void bp_dy(const DevPlan &P, d3 &x, d3 &u, double step, double q,
-                                      double m, Cand *cc) {
+__device__ __forceinline__ void bp_dy(const DevPlan &P, d3 &x, d3 &u, double step, const BorisFactors &f, Cand *cc) {
     x = add(x, divs(muls(u, step), 2.));
-    d3 B = field_at<FS>(P, x, cc);
-    d3 t = divs(muls(divs(divs(muls(B, q), 2), m), step), kCLight);
-    d3 s = divs(muls(t, 2), (1 + dot(t, t)));
-    d3 vh = add(u, cross(u, t));
-    u = add(u, cross(vh, s));
+    u = boris_rotate<false>(u, field_at<FS>(P, x, cc), step, f);
     x = add(x, divs(muls(u, step), 2.));
 }
 
@@ -426,8 +520,7 @@ __device__ __forceinline__ void neutral_step(const DevModule &m, Cand &c) {
 }
 
 __device__ __forceinline__ void set_direction(Cand &c, d3 uo) {
-    d3 u = unit(uo);
-    u = divs(u, norm(u));  // ParticleState::setDirection normalises again
+    const d3 u = unit_twice(uo);  // ParticleState::setDirection normalises again
     c.dx = u.x; c.dy = u.y; c.dz = u.z;
 }
 
@@ -456,10 +549,10 @@ struct BP {
     __device__ __forceinline__ static bool attempt(const DevPlan &P, const DevModule &m, Cand &c, Try &t,
                                                    StepCount &sc, bool on = true) {
         double step = t.step, newStep = step;
-        const double mass = c.E / (kCLight * kCLight);
+        const BorisFactors f(c.q, c.E);
         d3 xo = mk(c.x, c.y, c.z), uo = mk(c.dx, c.dy, c.dz);
         if (MODE == 1) {
-            bp_dy<FS>(P, xo, uo, step, c.q, mass, &c);
+            bp_dy<FS>(P, xo, uo, step, f, &c);
             if (!on) return false;
             sc.tries++; sc.evals++;
         } else {
@@ -468,7 +561,7 @@ struct BP {
             double h = step;
 #pragma unroll 1
             for (int i = 0; i < 3; i++) {
-                bp_dy<FS>(P, x, u, h, c.q, mass, &c);
+                bp_dy<FS>(P, x, u, h, f, &c);
                 if (i == 0) {
                     xo = x; uo = u;
                     x = mk(c.x, c.y, c.z); u = mk(c.dx, c.dy, c.dz);
@@ -493,93 +586,26 @@ struct BP {
     }
 };
 
-// ------------------------------------------- the same push without divisions
-// IEEE divisions and square roots make half of the push's instructions (eighteen
-// divisions and two square roots of 652).  Every one of them divides by
-// something known beforehand (the grid spacing, the candidate's mass, c), shared
-// by three components (1 + t^2) or within rounding of 1 (the norms), and the
-// same correctly rounded quotients follow from a correctly rounded reciprocal
-// by fused remainders:
-//
-// a / b, rounded to nearest, for rb = 1 / b rounded to nearest (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor",
-// 1990): the first correction leaves a quotient within one ulp, whose remainder
-// is exact, and the second rounds it correctly.  a and a / b nonzero and far
-// from the ends of the exponent range.
-__device__ __forceinline__ double quotient(double a, double b, double rb) {
-    double q = a * rb;
-    q = fma(fma(-q, b, a), rb, q);
-    return fma(fma(-q, b, a), rb, q);
-}
-__device__ __forceinline__ d3 quotient(d3 a, double b, double rb) {
-    return {quotient(a.x, b, rb), quotient(a.y, b, rb), quotient(a.z, b, rb)};
-}
-
-// u / |u| for n2 = u.u within 2^-27 of 1.  With n2 = 1 + e the square root is
-// 1 + e/2 - e^2/8, and e/2 is a multiple of half the spacing of doubles there:
-// the small last term only decides the ties, downwards, so rounding 1 + e/2 down
-// gives the correctly rounded root r.  In the same way 1/r = 1 - d + d^2 for
-// r = 1 + d is 2 - r with its ties rounded up.
-__device__ __forceinline__ d3 unit_near_1(d3 u, double n2) {
-    const double r = __fma_rd(0.5, n2, 0.5);
-    return quotient(u, r, __dsub_ru(2.0, r));
-}
-
-__device__ __forceinline__ int exponent_bits(double a) { return __double2hiint(a) & 0x7fffffff; }
-
 // The push of boris_body in the FP64 form: BP<FS_GRID_PERIODIC, 1>'s step, value
 // for value.
 struct BorisPush {
-    double q, mass, rmass;
+    BorisFactors f;
     unsigned tag;
     float corner[8][3];
-    // The range in which every quotient of bp_dy and its remainders are normal
-    // numbers, for any nonzero float field value.
     __device__ __forceinline__ static bool sane(const DevPlan &P, double q, double E) {
-        const double m = E / (kCLight * kCLight), step = P.modules[0].max_step;
-        return fabs(q) > 1e-60 && fabs(q) < 1e60 && m > 1e-60 && m < 1e60 && step > 1e-60 && step < 1e60;
+        return BorisFactors(q, E).plain && plain_step(P.modules[0].max_step);
     }
     __device__ __forceinline__ static double later(double time, double step) { return time + step / kCLight; }
-    __device__ __forceinline__ BorisPush(const DevPlan &P, double charge, double E) : q(charge) {
-        mass = E / (kCLight * kCLight);
-        rmass = 1.0 / mass;
-        tag = kNoCell;
-    }
+    __device__ __forceinline__ BorisPush(const DevPlan &, double q, double E) : f(q, E) { tag = kNoCell; }
     __device__ __forceinline__ void step(const DevPlan &P, double &x, double &y, double &z, double &ux, double &uy,
                                          double &uz) {
-        const DevGrid &g = P.fields[0].grid;
         const double h = P.modules[0].max_step;
         d3 X = mk(x, y, z), u = mk(ux, uy, uz);
         X = add(X, divs(muls(u, h), 2.));
-        const d3 B = grid_periodic(g, X, tag, corner);
-        d3 t, s;
-        double D;
-        const float least = fminf(fabsf((float)B.x), fminf(fabsf((float)B.y), fabsf((float)B.z)));
-        bool plain = least > 0.f;
-        if (plain) {
-            t = quotient(muls(quotient(divs(muls(B, q), 2), mass, rmass), h), kCLight, 1.0 / kCLight);
-            D = 1 + dot(t, t);
-            plain = D < 1e150;
-            s = quotient(muls(t, 2), D, 1.0 / D);
-        }
-        if (!plain) {  // a component is zero or not finite
-            t = divs(muls(divs(divs(muls(B, q), 2), mass), h), kCLight);
-            D = 1 + dot(t, t);
-            s = divs(muls(t, 2), D);
-        }
-        const d3 vh = add(u, cross(u, t));
-        u = add(u, cross(vh, s));
+        u = boris_rotate<true>(u, grid_periodic(P.fields[0].grid, X, tag, corner), h, f);
         X = add(X, divs(muls(u, h), 2.));
+        u = unit_twice(u);
         x = X.x; y = X.y; z = X.z;
-        const double n2 = u.x * u.x + u.y * u.y + u.z * u.z;
-        const int low = min(exponent_bits(u.x), min(exponent_bits(u.y), exponent_bits(u.z)));
-        if (fabs(n2 - 1) < 0x1p-27 && low > 0x07b00000) {  // every component above 2^-900
-            u = unit_near_1(u, n2);
-            u = unit_near_1(u, u.x * u.x + u.y * u.y + u.z * u.z);
-        } else {
-            u = unit(u);
-            u = divs(u, norm(u));
-        }
         ux = u.x; uy = u.y; uz = u.z;
     }
 };
@@ -602,6 +628,7 @@ __device__ __forceinline__ void ck_try(const DevPlan &P, d3 x, d3 u, double h, d
     d3 kx[6], ku[6];
     xo = x; uo = u;
     eu = mk(0, 0, 0);
+    const double qcE = q * kCLight / E;
 #pragma unroll
     for (int i = 0; i < 6; i++) {
         d3 yx = x, yu = u;
@@ -610,13 +637,15 @@ __device__ __forceinline__ void ck_try(const DevPlan &P, d3 x, d3 u, double h, d
             yx = add(yx, muls(muls(kx[j], ck_a[i * 6 + j]), h));
             yu = add(yu, muls(muls(ku[j], ck_a[i * 6 + j]), h));
         }
-        d3 vel = muls(unit(yu), kCLight);
+        d3 vel = muls(unit_fast(yu), kCLight);
         d3 B = field_at<FS>(P, yx, cc);
-        d3 dudt = muls(cross(vel, B), q * kCLight / E);
+        d3 dudt = muls(cross(vel, B), qcE);
         kx[i] = vel; ku[i] = dudt;
-        xo = add(xo, muls(muls(kx[i], ck_b[i]), h));
-        uo = add(uo, muls(muls(ku[i], ck_b[i]), h));
-        eu = add(eu, muls(muls(ku[i], ck_b[i] - ck_bs[i]), h));
+        if (i != 1 && i != 4) {  // b_1 = b_4 = 0
+            xo = add(xo, muls(muls(kx[i], ck_b[i]), h));
+            uo = add(uo, muls(muls(ku[i], ck_b[i]), h));
+        }
+        if (i != 1) eu = add(eu, muls(muls(ku[i], ck_b[i] - ck_bs[i]), h));
     }
 }
 

@@ -89,3 +89,43 @@ def test_device_fp64_against_golden(golden, name):
             np.testing.assert_array_equal(getattr(c, m), golden[f"{name}/out_{m}"], err_msg=m)
         for k, v in rec.sorted().items():
             np.testing.assert_array_equal(v, golden[f"{name}/rec_{k}"], err_msg=k)
+
+
+def test_correctly_rounded_pow_of_the_controllers(tmp_path):
+    """cr_pow (csrc/crmath.cuh) against 40-digit arithmetic: the quick evaluation
+    and the full one that takes over where it cannot round."""
+    import ctypes
+    import subprocess
+    from decimal import Decimal, localcontext
+    src = tmp_path / "p.cpp"
+    src.write_text('#include "crmath.cuh"\n'
+                   'extern "C" double cr(double x, double y) { return crp::cr_pow(x, y); }\n'
+                   'extern "C" int quick(double x, double y, double *r) { return crp::pow_quick(x, y, *r); }\n')
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC", "-w",
+                    "-I" + os.path.join(root, "crpropa3_b200", "csrc"), str(src), "-o", str(tmp_path / "p.so")],
+                   check=True)
+    lib = ctypes.CDLL(str(tmp_path / "p.so"))
+    lib.cr.restype = ctypes.c_double
+    lib.cr.argtypes = lib.quick.argtypes = [ctypes.c_double, ctypes.c_double]
+    lib.quick.argtypes = [ctypes.c_double, ctypes.c_double, ctypes.POINTER(ctypes.c_double)]
+    rng = np.random.default_rng(8)
+    x = np.concatenate([np.exp(rng.uniform(-12, 12, 600)), np.exp(rng.uniform(-690, 690, 200)),
+                        1 + rng.uniform(-1, 1, 200) * 2.0 ** rng.integers(-52, 0, 200), [0.5, 2.0, 1024.0, 1e-307]])
+    y = rng.choice([-0.2, 1 / 3, 0.5, 1.0, -1.0, 0.2371], len(x))
+    declined = 0
+    with localcontext() as ctx:
+        ctx.prec = 40
+        for a, b in zip(x.tolist(), y.tolist()):
+            value = (Decimal(a).ln() * Decimal(b)).exp()
+            exact = float(value)
+            if any(abs((Decimal(exact) + Decimal(float(np.nextafter(exact, to)))) / 2 - value) < value * 2 ** -98
+                   for to in (0.0, np.inf)):
+                continue  # closer to a midpoint than the evaluation's 100 bits tell
+            assert lib.cr(a, b) == exact, (a, b)
+            r = ctypes.c_double()
+            if lib.quick(a, b, ctypes.byref(r)):
+                assert r.value == exact, (a, b)
+            else:
+                declined += 1
+    assert declined < 0.05 * len(x)
