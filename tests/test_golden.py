@@ -119,7 +119,7 @@ def test_correctly_rounded_pow_of_the_controllers(tmp_path):
         for a, b in zip(x.tolist(), y.tolist()):
             value = (Decimal(a).ln() * Decimal(b)).exp()
             exact = float(value)
-            if any(abs((Decimal(exact) + Decimal(float(np.nextafter(exact, to)))) / 2 - value) < value * 2 ** -98
+            if any(abs((Decimal(exact) + Decimal(float(np.nextafter(exact, to)))) / 2 - value) < value * Decimal(2) ** -98
                    for to in (0.0, np.inf)):
                 continue  # closer to a midpoint than the evaluation's 100 bits tell
             assert lib.cr(a, b) == exact, (a, b)
