@@ -119,6 +119,28 @@ __device__ __forceinline__ void load_corner_pairs(const float *pairs, Index b00,
     load_pair<WIDE>(pairs + 8 * (size_t)(b11 + iz0), c[6], c[7]);
 }
 
+// Ask for the corners of the cell a candidate enters next (L1 prefetch), guessed
+// at its entry into a cell as the neighbour across the face a straight line at
+// its direction u meets first; f: its place in the cell.  A launch with few warps
+// per SM otherwise waits out the latency of L2 on every cell change.
+__device__ __forceinline__ void ask_next_cell(const DevGrid &g, int ix, int iy, int iz, float fx, float fy, float fz,
+                                              float ux, float uy, float uz) {
+    const float tx = __fdividef((ux > 0.f ? 1.f - fx : fx) * g.spacing_f[0], fabsf(ux));
+    const float ty = __fdividef((uy > 0.f ? 1.f - fy : fy) * g.spacing_f[1], fabsf(uy));
+    const float tz = __fdividef((uz > 0.f ? 1.f - fz : fz) * g.spacing_f[2], fabsf(uz));
+    if (tx <= ty && tx <= tz) ix = (ix + (ux > 0.f ? 1 : -1)) & (g.nx - 1);
+    else if (ty <= tz) iy = (iy + (uy > 0.f ? 1 : -1)) & (g.ny - 1);
+    else iz = (iz + (uz > 0.f ? 1 : -1)) & (g.nz - 1);
+    const unsigned sy = (unsigned)g.nz, sx = (unsigned)g.ny * (unsigned)g.nz;
+    const unsigned x0 = (unsigned)ix * sx, x1 = (unsigned)((ix + 1) & (g.nx - 1)) * sx;
+    const unsigned y0 = (unsigned)iy * sy, y1 = (unsigned)((iy + 1) & (g.ny - 1)) * sy;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float *p = g.pairs + 8 * (size_t)((k & 1 ? x1 : x0) + (k & 2 ? y1 : y0) + (unsigned)iz);
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+    }
+}
+
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11).
 __device__ __forceinline__ uint4 philox4x32_10(uint4 ctr, uint32_t k0, uint32_t k1) {
 #pragma unroll

@@ -284,6 +284,7 @@ crp_status build_grid(crp_plan *p, const crp_grid3f_desc &g, int comps, DevGrid 
     dg.goy = g.origin[1] + g.spacing[1] / 2;
     dg.goz = g.origin[2] + g.spacing[2] / 2;
     dg.sx = g.spacing[0]; dg.sy = g.spacing[1]; dg.sz = g.spacing[2];
+    for (int a = 0; a < 3; a++) dg.spacing_f[a] = (float)g.spacing[a];
     dg.inv_sx = 1.0 / g.spacing[0]; dg.inv_sy = 1.0 / g.spacing[1]; dg.inv_sz = 1.0 / g.spacing[2];
     dg.ox = g.origin[0]; dg.oy = g.origin[1]; dg.oz = g.origin[2];
     // edge = origin + Vector3d(Nx, Ny, Nz) * spacing (Grid.h:322)
@@ -718,6 +719,11 @@ crp_status crp_plan_create(const crp_plan_desc *desc, crp_plan **out) {
     }
     else if (d.n_fields == 1 && !desc->fields[0].periodic && desc->fields[0].kind == CRP_FIELD_PLANE_WAVE)
         p->fs = FS_PLANE_WAVE;
+    else if (d.n_fields == 1 && !desc->fields[0].periodic &&
+             (desc->fields[0].kind == CRP_FIELD_JF12 || desc->fields[0].kind == CRP_FIELD_UF23 ||
+              desc->fields[0].kind == CRP_FIELD_PT11 || desc->fields[0].kind == CRP_FIELD_TF17 ||
+              desc->fields[0].kind == CRP_FIELD_KST24))
+        p->fs = FS_GALACTIC;
     else
         p->fs = FS_GENERIC;
     crp_status st = ensure_counters(p);

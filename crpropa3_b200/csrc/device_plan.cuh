@@ -24,7 +24,8 @@ struct DevGrid {
     int pow2;              // nx, ny, nz all powers of two (periodic wrap by mask)
     double gox, goy, goz;  // gridOrigin = origin + spacing/2 (Grid.h:227)
     double sx, sy, sz;     // spacing
-    double inv_sx, inv_sy, inv_sz;  // 1/spacing (mixed form only)
+    double inv_sx, inv_sy, inv_sz;  // 1/spacing, rounded to nearest
+    float spacing_f[3];    // spacing, for guesses of the next cell
     double ox, oy, oz;     // origin (clipVolume test)
     double ex, ey, ez;     // origin + N*spacing (clipVolume test, Grid.h:322)
     int interp;            // crp_interpolation

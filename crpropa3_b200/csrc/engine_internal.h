@@ -15,6 +15,7 @@ enum FieldSig {
     FS_GENERIC = 0,    // any sum of (possibly periodic) components
     FS_GRID = 1,       // one MagneticFieldGrid, not wrapped
     FS_PLANE_WAVE = 2, // one PlaneWaveTurbulence, not wrapped
+    FS_GALACTIC = 5,   // one galactic field class (JF12, UF23, PT11, TF17, KST24), not wrapped
     FS_PLANE_WAVE_BLOCK = 4,  // FS_PLANE_WAVE, the mode sums shared by a block (chosen per launch)
     FS_GRID_PERIODIC = 3  // FS_GRID with a periodic grid of power-of-two dimensions, no
                           // clipVolume and with pair records: no runtime checks
@@ -50,6 +51,9 @@ inline int lanes_per_warp(uint64_t n, int num_sms, int warps_per_sm) {
     const uint64_t l = (n + warps - 1) / warps;
     return l < 1 ? 1 : l > 32 ? 32 : (int)l;
 }
+
+// Runs up to this size ask for the next grid cell ahead (step_*_bp.cu).
+constexpr uint64_t kAskAheadCandidates = 592 * 40;
 
 // Warps of candidates per block of a chunked launch over a PlaneWaveTurbulence
 // field evaluated by the block: the fewest whose blocks are resident at once (592:

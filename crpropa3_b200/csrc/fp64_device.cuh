@@ -43,6 +43,12 @@
 #ifndef CRP_BP_GRID_MIN_BLOCKS
 #define CRP_BP_GRID_MIN_BLOCKS 4
 #endif
+// The adaptive Boris push: 3 blocks (50 000 candidates over a 100^3 grid, mixed:
+// 2.32 ms at the 2 its 195 registers allowed, 1.43 ms at 3, 1.58 at 4 with spills;
+// FP64 3.1, 2.1 and 2.4 ms).
+#ifndef CRP_BP_ADAPTIVE_MIN_BLOCKS
+#define CRP_BP_ADAPTIVE_MIN_BLOCKS 3
+#endif
 #ifndef CRP_CK_MIN_BLOCKS
 #define CRP_CK_MIN_BLOCKS 3
 #endif
@@ -165,7 +171,8 @@ __device__ __forceinline__ d3 trilinear(const float (&c)[8][3], double fX0, doub
 // coordinates are quotients by the spacing (g.inv_s*: its correctly rounded
 // reciprocal); where one is too small for an exact remainder its cell and
 // single-precision fraction do not depend on the last bit.
-__device__ __forceinline__ d3 grid_periodic(const DevGrid &g, d3 pos, unsigned &tag, float (&corner)[8][3]) {
+template <bool AHEAD>
+__device__ __forceinline__ d3 grid_periodic(const DevGrid &g, d3 pos, unsigned &tag, float (&corner)[8][3], d3 u) {
     const double rx = quotient(pos.x - g.gox, g.sx, g.inv_sx), ry = quotient(pos.y - g.goy, g.sy, g.inv_sy),
                  rz = quotient(pos.z - g.goz, g.sz, g.inv_sz);
     const CellIndex i = cell_index(rx, ry, rz);
@@ -176,6 +183,9 @@ __device__ __forceinline__ d3 grid_periodic(const DevGrid &g, d3 pos, unsigned &
         const unsigned x1 = (unsigned)((ix0 + 1) & (g.nx - 1)) * sx, y1 = (unsigned)((iy0 + 1) & (g.ny - 1)) * sy;
         load_corner_pairs<true>(g.pairs, x0 + y0, x1 + y0, x0 + y1, x1 + y1, iz0, corner);
         tag = x0 + y0 + iz0;
+        if (AHEAD)
+            ask_next_cell(g, ix0, iy0, iz0, (float)(rx - i.flx), (float)(ry - i.fly), (float)(rz - i.flz), (float)u.x,
+                          (float)u.y, (float)u.z);
     }
     return trilinear(corner, rx - i.flx, ry - i.fly, rz - i.flz);
 }
@@ -451,12 +461,26 @@ __device__ __noinline__ d3 field_sum(const DevComponent *f, int n, d3 pos) {
     return b;
 }
 
+// A single galactic field, without the sum's tests and loads.
+__device__ __forceinline__ d3 galactic_field(const DevComponent &f, d3 pos) {
+    u3 b;
+    switch (f.kind) {
+    case CRP_FIELD_JF12: return jf12_field(f, pos);
+    case CRP_FIELD_UF23: b = uf23_field(*f.uf, pos.x, pos.y, pos.z); break;
+    case CRP_FIELD_PT11: b = pt11_field(*f.pt, pos.x, pos.y, pos.z); break;
+    case CRP_FIELD_TF17: b = tf17_field(*f.tf, pos.x, pos.y, pos.z); break;
+    default: b = kst24_field(*f.kst, pos.x, pos.y, pos.z);
+    }
+    return mk(b.x, b.y, b.z);
+}
+
 template <int FS>
 __device__ __forceinline__ d3 field_at(const DevPlan &P, d3 pos, Cand *cc = nullptr) {
     if (FS == FS_GRID) return grid_field_t<true>(P.fields[0].grid, pos, cc);
     if (FS == FS_GRID_PERIODIC) return grid_field_t<true, true>(P.fields[0].grid, pos, cc);
     if (FS == FS_PLANE_WAVE) return plane_wave_field(P.fields[0].pw, pos);
     if (FS == FS_PLANE_WAVE_BLOCK) return plane_wave_block(P.fields[0].pw, pos, P.block_warps);
+    if (FS == FS_GALACTIC) return galactic_field(P.fields[0], pos);
     return field_sum(P.dev_fields, P.n_fields, pos);
 }
 
@@ -587,8 +611,10 @@ struct BP {
 };
 
 // The push of boris_body in the FP64 form: BP<FS_GRID_PERIODIC, 1>'s step, value
-// for value.
+// for value.  AHEAD: ask_next_cell.
+template <bool AHEAD>
 struct BorisPush {
+    static constexpr bool kAhead = AHEAD;
     BorisFactors f;
     unsigned tag;
     float corner[8][3];
@@ -602,7 +628,7 @@ struct BorisPush {
         const double h = P.modules[0].max_step;
         d3 X = mk(x, y, z), u = mk(ux, uy, uz);
         X = add(X, divs(muls(u, h), 2.));
-        u = boris_rotate<true>(u, grid_periodic(P.fields[0].grid, X, tag, corner), h, f);
+        u = boris_rotate<true>(u, grid_periodic<AHEAD>(P.fields[0].grid, X, tag, corner, u), h, f);
         X = add(X, divs(muls(u, h), 2.));
         u = unit_twice(u);
         x = X.x; y = X.y; z = X.z;
@@ -835,7 +861,7 @@ template <int FS> using BPFixed = BP<FS, 1>;
 // the fixed-step Boris push is latency bound on its gathers and wants warps
 template <class T> struct MinBlocks { static constexpr int value = 1; };
 template <int FS, int MODE> struct MinBlocks<BP<FS, MODE>> {
-    static constexpr int value = MODE != 1 ? 1 : FS == FS_GRID ? CRP_BP_GRID_MIN_BLOCKS : CRP_BP_FIXED_MIN_BLOCKS;
+    static constexpr int value = MODE != 1 ? CRP_BP_ADAPTIVE_MIN_BLOCKS : FS == FS_GRID ? CRP_BP_GRID_MIN_BLOCKS : CRP_BP_FIXED_MIN_BLOCKS;
 };
 template <int FS, int MODE> struct MinBlocks<CK<FS, MODE>> { static constexpr int value = CRP_CK_MIN_BLOCKS; };
 template <int FS> using BPAdaptive = BP<FS, 2>;
@@ -861,9 +887,9 @@ __global__ void __launch_bounds__(128, MinBlocks<Prop<FS>>::value) fp64_persiste
 }
 
 // The kernel of a field signature and chain shape: compiled chain shapes for
-// the single-field signatures and, for the backtracking chain [propagation,
-// MaximumTrajectoryLength, Observer], the generic field sum; otherwise the
-// module list is walked.
+// the single-field signatures (galactic fields: the backtracking chain
+// [propagation, MaximumTrajectoryLength, Observer]); otherwise the module list is
+// walked.
 template <class F>
 void for_signature(int fs, int shape, F f) {
     using std::integral_constant;
@@ -882,10 +908,12 @@ void for_signature(int fs, int shape, F f) {
         if (shape == CS_PM) f(s, pm);
         else if (shape == CS_PMO) f(s, pmo);
         else f(s, any);
-    } else {
-        integral_constant<int, FS_GENERIC> s;
+    } else if (fs == FS_GALACTIC) {
+        integral_constant<int, FS_GALACTIC> s;
         if (shape == CS_PMO) f(s, pmo);
         else f(s, any);
+    } else {
+        f(integral_constant<int, FS_GENERIC>(), any);
     }
 }
 
@@ -896,7 +924,7 @@ void for_signature(int fs, int shape, F f) {
 // candidates x 1500 steps over 64^3: 3.54 ms, then 1.49, 1.55 and 1.98 ms).
 constexpr int kBorisMinBlocks = 4;
 template <class Push>
-__global__ void __launch_bounds__(128, kBorisMinBlocks)
+__global__ void __launch_bounds__(128, Push::kAhead ? 4 : kBorisMinBlocks)
 fp64_boris_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, int lanes, int max_steps, uint64_t step_cap,
                    DevCounters *cnt, DevRecords rec, const uint32_t *perm, uint32_t *perm_out) {
     boris_body<Push, BPFixed<FS_GRID_PERIODIC>>(P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);

@@ -43,6 +43,12 @@
 #ifndef CRP_BP_GRID_MIN_BLOCKS
 #define CRP_BP_GRID_MIN_BLOCKS 4
 #endif
+// The adaptive Boris push: 3 blocks (50 000 candidates over a 100^3 grid, mixed:
+// 2.32 ms at the 2 its 195 registers allowed, 1.43 ms at 3, 1.58 at 4 with spills;
+// FP64 3.1, 2.1 and 2.4 ms).
+#ifndef CRP_BP_ADAPTIVE_MIN_BLOCKS
+#define CRP_BP_ADAPTIVE_MIN_BLOCKS 3
+#endif
 #ifndef CRP_CK_MIN_BLOCKS
 #define CRP_CK_MIN_BLOCKS 3
 #endif
@@ -81,8 +87,9 @@ __device__ __forceinline__ int wrap(int i, int n, bool pow2) {
 // the cache.
 struct CellFrac { float fx0, fy0, fz0; };
 
+template <bool AHEAD = false>
 __device__ __forceinline__ CellFrac grid_cell_load(const DevGrid &g, double x, double y, double z, unsigned &tag,
-                                                   float (&corner)[8][3]) {
+                                                   float (&corner)[8][3], double ux = 0, double uy = 0, double uz = 0) {
     const double rx = (x - g.gox) * g.inv_sx, ry = (y - g.goy) * g.inv_sy, rz = (z - g.goz) * g.inv_sz;
     const CellIndex c = cell_index(rx, ry, rz);
     const CellFrac f{(float)__dsub_rn(rx, c.flx), (float)__dsub_rn(ry, c.fly), (float)__dsub_rn(rz, c.flz)};
@@ -96,6 +103,7 @@ __device__ __forceinline__ CellFrac grid_cell_load(const DevGrid &g, double x, d
         const unsigned x0 = (unsigned)ix0 * sx, y0 = (unsigned)iy0 * sy;
         load_corner_pairs<true>(g.pairs, b00, x1 + y0, x0 + y1, x1 + y1, iz0, corner);
         tag = b00 + iz0;
+        if (AHEAD) ask_next_cell(g, ix0, iy0, iz0, f.fx0, f.fy0, f.fz0, (float)ux, (float)uy, (float)uz);
     }
     return f;
 }
@@ -1087,6 +1095,18 @@ __device__ __noinline__ f3 field_sum(const DevComponent *f, int n, double x, dou
     return b;
 }
 
+// A single galactic field, called without the sum's tests and loads (each some
+// 35 cycles of latency per field in chains that have one warp per scheduler).
+__device__ __forceinline__ f3 galactic_field(const DevComponent &f, double x, double y, double z) {
+    switch (f.kind) {
+    case CRP_FIELD_JF12: return jf12_field_f(f, x, y, z);
+    case CRP_FIELD_UF23: return uf23_field_f(f, x, y, z);
+    case CRP_FIELD_PT11: return pt11_field_f(f, x, y, z);
+    case CRP_FIELD_TF17: return tf17_field_f(f, x, y, z);
+    default: return kst24_field_f(f, x, y, z);
+    }
+}
+
 template <int FS, bool FUSED = false>
 __device__ __forceinline__ f3 field_at(const DevPlan &P, double x, double y, double z,
                                        Cand *cc = nullptr, const PwTab *sh = nullptr) {
@@ -1094,6 +1114,7 @@ __device__ __forceinline__ f3 field_at(const DevPlan &P, double x, double y, dou
     if (FS == FS_GRID_PERIODIC) return grid_field_t<true, true>(P.fields[0].grid, x, y, z, cc);
     if (FS == FS_PLANE_WAVE) return plane_wave_field(P.fields[0].pw, x, y, z, sh);
     if (FS == FS_PLANE_WAVE_BLOCK) return plane_wave_block(P.fields[0].pw, x, y, z, P.block_warps);
+    if (FS == FS_GALACTIC) return galactic_field(P.fields[0], x, y, z);
     return field_sum(P.dev_fields, P.n_fields, x, y, z, sh);
 }
 
@@ -1223,7 +1244,10 @@ struct BP {
 };
 
 // The push of boris_body in the mixed form: BP<FS_GRID_PERIODIC, 1>'s step.
+// AHEAD: ask_next_cell.
+template <bool AHEAD>
 struct BorisPush {
+    static constexpr bool kAhead = AHEAD;
     float kt;
     unsigned tag;
     float corner[8][3];
@@ -1237,7 +1261,7 @@ struct BorisPush {
                                          double &uz) {
         const double hh = 0.5 * P.modules[0].max_step;
         x = fma(ux, hh, x); y = fma(uy, hh, y); z = fma(uz, hh, z);
-        const CellFrac f = grid_cell_load(P.fields[0].grid, x, y, z, tag, corner);
+        const CellFrac f = grid_cell_load<AHEAD>(P.fields[0].grid, x, y, z, tag, corner, ux, uy, uz);
         bp_rotate_drift(x, y, z, ux, uy, uz, grid_cell_interp(f, corner), kt, hh);
         renorm(ux, uy, uz);
     }
@@ -1593,7 +1617,7 @@ template <int FS> using BPFixed = BP<FS, 1>;
 // the fixed-step Boris push is latency bound on its gathers and wants warps
 template <class T> struct MinBlocks { static constexpr int value = 1; };
 template <int FS, int MODE> struct MinBlocks<BP<FS, MODE>> {
-    static constexpr int value = MODE != 1 ? 1 : FS == FS_GRID ? CRP_BP_GRID_MIN_BLOCKS : CRP_BP_FIXED_MIN_BLOCKS;
+    static constexpr int value = MODE != 1 ? CRP_BP_ADAPTIVE_MIN_BLOCKS : FS == FS_GRID ? CRP_BP_GRID_MIN_BLOCKS : CRP_BP_FIXED_MIN_BLOCKS;
 };
 template <int FS, int MODE> struct MinBlocks<CK<FS, MODE>> { static constexpr int value = CRP_CK_MIN_BLOCKS; };
 template <int FS> using BPAdaptive = BP<FS, 2>;
@@ -1619,9 +1643,9 @@ __global__ void __launch_bounds__(128, MinBlocks<Prop<FS>>::value) mixed_persist
 }
 
 // The kernel of a field signature and chain shape: compiled chain shapes for
-// the single-field signatures and, for the backtracking chain [propagation,
-// MaximumTrajectoryLength, Observer], the generic field sum; otherwise the
-// module list is walked.
+// the single-field signatures (galactic fields: the backtracking chain
+// [propagation, MaximumTrajectoryLength, Observer]); otherwise the module list is
+// walked.
 template <class F>
 void for_signature(int fs, int shape, F f) {
     using std::integral_constant;
@@ -1640,10 +1664,12 @@ void for_signature(int fs, int shape, F f) {
         if (shape == CS_PM) f(s, pm);
         else if (shape == CS_PMO) f(s, pmo);
         else f(s, any);
-    } else {
-        integral_constant<int, FS_GENERIC> s;
+    } else if (fs == FS_GALACTIC) {
+        integral_constant<int, FS_GALACTIC> s;
         if (shape == CS_PMO) f(s, pmo);
         else f(s, any);
+    } else {
+        f(integral_constant<int, FS_GENERIC>(), any);
     }
 }
 
@@ -1654,7 +1680,7 @@ void for_signature(int fs, int shape, F f) {
 // 45.3 at 8; 20 011 candidates x 1000 steps: 0.80, 0.80 and 0.85 ms).
 constexpr int kBorisMinBlocks = 7;
 template <class Push>
-__global__ void __launch_bounds__(128, kBorisMinBlocks)
+__global__ void __launch_bounds__(128, Push::kAhead ? 4 : kBorisMinBlocks)
 mixed_boris_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, int lanes, int max_steps, uint64_t step_cap,
                    DevCounters *cnt, DevRecords rec, const uint32_t *perm, uint32_t *perm_out) {
     boris_body<Push, BPFixed<FS_GRID_PERIODIC>>(P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);

@@ -14,8 +14,16 @@ cudaError_t launch_fp64_bp_chunk(const DevPlan &P, const DevState &s, uint64_t n
     const bool fixed = pm.min_step == pm.max_step;
     if (fixed && fs == FS_GRID_PERIODIC && P.shape == CS_PM) {
         const uint64_t slots = (uint64_t)(block / 32) * (uint64_t)lanes;
-        fp64_boris_kernel<BorisPush><<<(unsigned)((n + slots - 1) / slots), block, 0, st>>>(
-            P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
+        const unsigned grid = (unsigned)((n + slots - 1) / slots);
+        // about one warp per scheduler or less (40 candidates for each): nothing else
+        // hides the gathers' latency (256^3 grid, 1000 steps, mixed: 2000 candidates
+        // 0.81 -> 0.68 ms, 20 011 0.79 -> 0.76 ms; 50 000 lose, 1.02 -> 1.19 ms)
+        if (n <= kAskAheadCandidates)
+            fp64_boris_kernel<BorisPush<true>><<<grid, block, 0, st>>>(
+                P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
+        else
+            fp64_boris_kernel<BorisPush<false>><<<grid, block, 0, st>>>(
+                P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
         return cudaGetLastError();
     }
     return fixed ? launch_prop<BPFixed>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, lanes, st)

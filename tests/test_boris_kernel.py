@@ -67,9 +67,9 @@ def test_fp64_matches_the_oracle(oracle, n, per_candidate, steps_per_launch):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", [_abi.PRECISION_FP64, _abi.PRECISION_MIXED])
-@pytest.mark.parametrize("cap", [0, 1, 130])
-def test_same_as_the_module_list_kernel(precision, cap):
-    c = _candidates(701)
+@pytest.mark.parametrize("n,cap", [(701, 0), (701, 1), (701, 130), (24001, 0)])  # with and without asking ahead
+def test_same_as_the_module_list_kernel(precision, n, cap):
+    c = _candidates(n)
     a, ra, sa = _run(_spec(precision), c, max_steps=cap)
     b, rb, sb = _run(_spec(precision, extra=True), c, max_steps=cap)
     for name in NAMES:
