@@ -41,7 +41,7 @@ import numpy as np  # noqa: E402
 METRIC = "particle-steps/s, 1 B200: mixed-prec vs FP64 at stated error; adjoint cost/fwd"
 UNIT = "particle-steps/s"
 ALGO_BYTES_PER_STEP = 96  # 8 corners x 12 B Grid3f payload per field evaluation
-TRAFFIC_B_PER_STEP = 13.65  # DRAM read+write per particle-step of the mixed kernel (ncu, all launches of a full run)
+TRAFFIC_B_PER_STEP = 20.16  # DRAM read+write per particle-step of the mixed kernel (ncu, all launches of a full run)
 
 
 def log(*a):
@@ -445,9 +445,8 @@ def cfg_grid_ck_64(dev, peaks, n=10_000):
         out.setdefault("grid_ck_64", {
             "workload": f"{n} protons 1-100 EeV, 64^3 Grid3f 1 nG 10 kpc, PropagationCK 1e-4 "
                         "0.1-10 kpc, MaximumTrajectoryLength 10 Mpc, full runs",
-            "note": "10^4 candidates are 79 blocks of 128 (one thread per candidate); the run time is "
-                    "the serial step chain of the slowest candidates: spreading them over all 148 SMs "
-                    "in single-warp blocks measured no faster (4.24e9 vs 4.20e9 tries/s)"})[name] = {
+            "note": "10^4 candidates are one warp of 17 per scheduler (one thread per candidate); the "
+                    "run time is a warp's serial chain of steps"})[name] = {
             "tries_per_s": tries_s, "particle_steps_per_s": t["particle_steps"] / (t["device_ms"] / 1e3),
             "ms_per_run": t["device_ms"] / 3,
             "roofline": {"bound": "l2", "achieved": gbs, "peak": peaks.get("l2_gbs"), "unit": "GB/s",
@@ -760,13 +759,13 @@ def main():
 
     # every stepping launch of the process, per form, for comparison with the
     # ncu launch list of the same command
-    MIXED_KERNEL = "mixed_chunk_kernel<BPFixed>"
-    kernel_time = {MIXED_KERNEL: [0, 0.0], "fp64_chunk_kernel<BPFixed>": [0, 0.0]}
+    MIXED_KERNEL = "mixed_boris_kernel"
+    kernel_time = {MIXED_KERNEL: [0, 0.0], "fp64_boris_kernel": [0, 0.0]}
 
     def one_step(plan):
         reset()
         st = plan.run(d_work)
-        k = kernel_time[MIXED_KERNEL if plan is plan_mx else "fp64_chunk_kernel<BPFixed>"]
+        k = kernel_time[MIXED_KERNEL if plan is plan_mx else "fp64_boris_kernel"]
         k[0] += st.launches
         k[1] += st.device_ms
         return st

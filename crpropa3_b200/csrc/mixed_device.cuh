@@ -1,8 +1,8 @@
 // mixed_device.cuh -- device code of the mixed-precision form shared by its
-// translation units (step_mixed.cu, step_mixed_bp.cu): field evaluation,
+// translation units (step_mixed.cu, step_mixed_bp.cu, step_mixed_ck.cu): field evaluation,
 // the propagation modules and the chunked stepping kernel template.
 //
-// Same modules and module order as the FP64 form (step_fp64.cu), with the
+// Same modules and module order as the FP64 form (fp64_device.cuh), with the
 // arithmetic split by what each quantity needs:
 //   * FP64: position, trajectory length, time, the step controller's error
 //     sum and its pow(), grid coordinates before the cell split, wave phases
@@ -80,7 +80,7 @@ __device__ __forceinline__ int wrap(int i, int n, bool pow2) {
 // With a cell cache (FS_GRID kernels) the 8 corners are loaded only when the
 // cell changes.
 // PER: the grid is periodic with power-of-two dimensions, has no clipVolume
-// and has the padded copy (FS_GRID_PERIODIC): those branches are compiled out.
+// and has pair records (FS_GRID_PERIODIC): those branches are compiled out.
 // The periodic power-of-two case in two parts: grid_cell_load finds the
 // cell of (x, y, z) and, when it is not the cached one, loads its 8 corners
 // into the candidate's cache; grid_cell_interp forms the trilinear sum from
