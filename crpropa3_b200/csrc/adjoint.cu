@@ -20,6 +20,7 @@
 // oracle's CPU adjoint (which divides) to rounding, not bit for bit.
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <type_traits>
@@ -541,7 +542,8 @@ static crp_status adjoint_impl(const crp_adjoint_desc *d, const crp_adjoint_io *
     unsigned long long *acc = reinterpret_cast<unsigned long long *>(w + align256(256) + align256(nck * 6 * a->n * sizeof(double)));
     AdjGrid G = make_grid(d);
     const size_t cells = cells3 / 3;
-    if (cells <= kPairCells)
+    // (a workspace off the records' 32-byte alignment reads the grid in place)
+    if (cells <= kPairCells && reinterpret_cast<uintptr_t>(workspace) % 32 == 0)
         G.pairs = reinterpret_cast<const float *>(reinterpret_cast<char *>(acc) + align256(cells3 * sizeof(unsigned long long)));
     const IO io = make_io(a);
     auto blocks = [&](unsigned threads) { return (unsigned)((a->n + threads - 1) / threads); };

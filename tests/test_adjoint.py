@@ -141,3 +141,31 @@ def test_adjoint_of_directions_off_unit_length(oracle):
     got = _gpu(grid, pos, u0, energy, charge, target)
     for g, r, tol in zip(got, ref, (1e-12, 1e-10, 1e-10, 1e-9)):
         np.testing.assert_allclose(g, r, rtol=0, atol=tol * np.abs(r).max())
+
+
+def test_adjoint_in_a_workspace_of_any_alignment():
+    """The pair records want 32 bytes; a workspace off that reads the grid in place, with the same bits."""
+    import ctypes as C
+    import torch
+    from crpropa3_b200 import _abi
+    from crpropa3_b200.adjoint import _desc, _io, _planar
+    grid, pos, u0, energy, charge, target = _problem(n=40, seed=86)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    g, lib = t(grid), _abi.load()
+    d = _desc(g, ORIGIN, SPACING, STEP, NSTEPS, K)
+    need = C.c_size_t()
+    _abi.check(lib.crp_bp_adjoint_workspace(C.byref(d), 40, C.byref(need)))
+    ins = [_planar(t(a)) for a in (pos, u0, target)]
+    e, q = t(energy), t(charge)
+    got = []
+    for offset in (0, 8):
+        ws = torch.empty(need.value + 64, dtype=torch.uint8, device="cuda")
+        loss, ge = torch.empty(40, dtype=torch.float64, device="cuda"), torch.empty(40, dtype=torch.float64, device="cuda")
+        gu = [torch.empty_like(loss) for _ in range(3)]
+        gg = torch.empty(g.shape, dtype=torch.float64, device="cuda")
+        io = _io(40, ins[0], ins[1], e, q, ins[2], loss, None, gu, ge, gg)
+        _abi.check(lib.crp_bp_adjoint(C.byref(d), C.byref(io), C.c_void_p(ws.data_ptr() + offset), need.value, None))
+        torch.cuda.synchronize()
+        got.append([a.cpu().numpy() for a in (loss, *gu, ge, gg)])
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)
