@@ -64,11 +64,20 @@ constexpr uint64_t kAskAheadCandidates = 592 * 40;
 // 10^5 candidates, 100 modes: 1.50 ms thread by thread, 2.07 ms by blocks;
 // 20 000 candidates, 200 modes: 5.16 and 4.06 ms; the mixed form 4 x 10^5
 // candidates, 300 modes: 7.08 and 3.92 ms, 20 modes: 0.86 and 0.82 ms).
+constexpr int kWaveMaxModes = 1365;
 inline int wave_block_warps(uint64_t n, int n_modes, bool fp64) {
-    if (n_modes < (fp64 ? 32 : 8) || n_modes > 1365) return 0;
+    if (n_modes < (fp64 ? 32 : 8) || n_modes > kWaveMaxModes) return 0;
     if (n <= 592u * 32u) return 1;
     if (n <= 592u * 64u) return 2;
     return fp64 ? 0 : 4;
+}
+
+// Dynamic shared memory a kernel may be launched with: MOST, the largest that
+// any plan asks of it.  The limit belongs to the kernel, not to a launch: setting
+// it to one plan's table would lower it under another thread's launch.
+template <size_t MOST, class Kernel>
+inline cudaError_t allow_shared(Kernel kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST);
 }
 
 // step_fp64.cu

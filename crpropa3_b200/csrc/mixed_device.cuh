@@ -1709,8 +1709,7 @@ cudaError_t launch_waves(DevPlan P, const DevState &s, uint64_t n, int max_steps
     const unsigned grid = (unsigned)((n + 32 * warps - 1) / (32 * warps));
     auto launch = [&](auto c) {
         auto kernel = mixed_wave_kernel<Prop, decltype(c)::value>;
-        // beside the kernel's own shared memory
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_shared<(size_t)((kWaveMaxModes + 1) / 2) * 80>(kernel);
         if (e != cudaSuccess) return e;
         kernel<<<grid, kBatchThreads, smem, st>>>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out);
         return cudaGetLastError();

@@ -249,22 +249,22 @@ cudaError_t launch_mixed_chunk(const DevPlan &P, const DevState &s, uint64_t n, 
     int pw_field = -1, n_pw = 0;
     for (int f = 0; f < P.n_fields; f++)
         if (P.fields[f].kind == CRP_FIELD_PLANE_WAVE) { pw_field = f; n_pw++; }
+    constexpr size_t most = 96 * 1024;
     size_t smem = 0;
-    if (n_pw == 1 && (size_t)P.fields[pw_field].pw.npairs * 80 <= 96 * 1024)
+    if (n_pw == 1 && (size_t)P.fields[pw_field].pw.npairs * 80 <= most)
         smem = (size_t)P.fields[pw_field].pw.npairs * 80;
     else
         pw_field = -1;
     if (pw_field >= 0 && (fs == FS_PLANE_WAVE || fs == FS_GENERIC)) {
         // block-batched plane-wave sums: the table, the block's query positions,
         // the four group sums per query and the warp counts
-        const size_t bsmem = smem + 3 * kBatchThreads * sizeof(double) +
-                             kPwGroups * 3 * kBatchThreads * sizeof(float) + 4 * sizeof(int);
+        constexpr size_t queries = 3 * kBatchThreads * sizeof(double) +
+                                   kPwGroups * 3 * kBatchThreads * sizeof(float) + 4 * sizeof(int);
+        const size_t bsmem = smem + queries;
         const unsigned bgrid = (unsigned)((n + kBatchThreads - 1) / kBatchThreads);
 #define CRP_SDE_BATCH(FSV)                                                                               \
     do {                                                                                                 \
-        if (bsmem > 48 * 1024)                                                                           \
-            cudaFuncSetAttribute(mixed_sde_batch_kernel<FSV>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                 (int)bsmem);                                                            \
+        if (bsmem > 48 * 1024) allow_shared<most + queries>(mixed_sde_batch_kernel<FSV>);                \
         mixed_sde_batch_kernel<FSV><<<bgrid, kBatchThreads, bsmem, st>>>(P, s, n, max_steps, step_cap, cnt, \
                                                                         rec, perm, perm_out, pw_field);  \
     } while (0)
@@ -275,9 +275,7 @@ cudaError_t launch_mixed_chunk(const DevPlan &P, const DevState &s, uint64_t n, 
     }
 #define CRP_SDE_COOP(FSV)                                                                              \
     do {                                                                                               \
-        if (smem > 48 * 1024)                                                                          \
-            cudaFuncSetAttribute(mixed_sde_coop_kernel<FSV>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                 (int)smem);                                                           \
+        if (smem > 48 * 1024) allow_shared<most>(mixed_sde_coop_kernel<FSV>);                          \
         mixed_sde_coop_kernel<FSV><<<grid, block, smem, st>>>(P, s, n, max_steps, step_cap, cnt, rec,  \
                                                               perm, perm_out, pw_field);               \
     } while (0)
