@@ -85,8 +85,8 @@ constexpr double kTurnScale = 4294967296.0;          // 2^32: turns as 32-bit fi
 // for runs of at least kPipelineMinCandidates
 constexpr int kInputChunks = 8;
 constexpr uint64_t kPipelineMinCandidates = 1u << 18;
-// crp_run() up to this size gathers its arrays in one pinned buffer: one copy in
-// and one out instead of 20 and 16 (257 candidates x 64 steps, FP64: 376 us with
+// crp_run() up to this size gathers pageable arrays in one pinned buffer: one copy
+// in and one out instead of 20 and 16 (257 candidates x 64 steps, FP64: 376 us with
 // separate copies, 144 us here)
 constexpr uint64_t kStagedCandidates = 1u << 15;
 
@@ -1261,7 +1261,15 @@ crp_status crp_run(crp_plan *p, const crp_candidates *h, uint64_t n, const crp_r
         CUDA_TRY(cudaStreamWaitEvent(p->copy_stream, p->ev_ready, 0));
         cs = p->copy_stream;
     }
-    const bool staged = n <= kStagedCandidates;
+    // Pageable arrays only: the runtime orders the copies of pinned and managed ones
+    // after what the stream (NULL: every blocking stream) has queued on them, and
+    // copies or refuses device memory itself.  (Asking costs 0.1 us per array.)
+    bool staged = n <= kStagedCandidates;
+    for (int k = 0; k < n_members && staged; k++) {
+        cudaPointerAttributes a{};
+        staged = cudaPointerGetAttributes(&a, members[k].host) == cudaSuccess && a.type == cudaMemoryTypeUnregistered;
+    }
+    cudaGetLastError();
     HostRun host{pipe ? &chunks : nullptr, nullptr, nullptr, 0, false};
     if (staged) {
         if (p->staging_bytes < off) {
