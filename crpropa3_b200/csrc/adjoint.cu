@@ -20,10 +20,8 @@
 // oracle's CPU adjoint (which divides) to rounding, not bit for bit.
 #include <cuda_runtime.h>
 
-#include <cstdint>
 #include <cstdio>
 #include <cstring>
-#include <type_traits>
 
 #include "crp_gpu.h"
 #include "engine_internal.h"
@@ -51,29 +49,10 @@ struct AdjGrid {
     bool pow2;  // every dimension a power of two: indices wrap with a mask
     double gox, goy, goz, sx, sy, sz;
     double isx, isy, isz;  // 1 / spacing
-    const float *pairs;    // pair records of the values (load_corners), or null
 };
 
-// The pair records are built for grids of up to 2^28 cells (8 GB of
-// workspace); larger grids are read in place.
-constexpr size_t kPairCells = (size_t)1 << 28;
-
-__global__ void pair_kernel(const float *g, int nz, unsigned cells, float4 *pairs) {
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cells) return;
-    const unsigned j = i % (unsigned)nz == (unsigned)nz - 1 ? i - (unsigned)(nz - 1) : i + 1;
-    const float *a = g + 3 * (size_t)i, *b = g + 3 * (size_t)j;
-    pairs[2 * (size_t)i] = make_float4(__ldg(a), __ldg(a + 1), __ldg(a + 2), 0.f);
-    pairs[2 * (size_t)i + 1] = make_float4(__ldg(b), __ldg(b + 1), __ldg(b + 2), 0.f);
-}
-
-// one 32-byte record in one aligned 256-bit load
-__device__ __forceinline__ void load_pair(const float *p, float a[3], float b[3]) {
-    float pad0, pad1;
-    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(pad0), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(pad1)
-                 : "l"(p));
-}
+// Grids below this take 32-bit linear indices (3 * cell + component < 2^32).
+constexpr size_t kSmallGrid = (size_t)1 << 30;
 
 // periodic index: i mod n in [0, n) (a mask for power-of-two n, the same value)
 __device__ __forceinline__ int wrap_index(int i, int n, bool pow2) {
@@ -125,8 +104,7 @@ __device__ __forceinline__ constexpr int bit(int q, int a) {
     return t[q][a];
 }
 
-// linear indices of the 8 corners, 32-bit with the pair records (at most
-// kPairCells cells)
+// linear indices of the 8 corners
 template <class Index>
 __device__ __forceinline__ void corner_indices(const AdjGrid &G, const int lo[3], Index idx[8]) {
     const Index sx = (Index)G.ny * (Index)G.nz, sy = (Index)G.nz;
@@ -147,27 +125,15 @@ struct Corners {
     float v[8][3];
 };
 
-// PAIRS: the grid's copy in pair records, 32 bytes per cell holding the
-// cell's value and its upper z neighbour's, so that a cell's corners are four
-// aligned 256-bit loads instead of 24 scalar ones.
-template <bool PAIRS>
+template <class Index>
 __device__ __forceinline__ void load_corners(const AdjGrid &G, const CellPos &c, Corners &k) {
     if (c.lo[0] == k.lo[0] && c.lo[1] == k.lo[1] && c.lo[2] == k.lo[2]) return;
-    if (PAIRS) {
-        unsigned idx[8];
-        corner_indices(G, c.lo, idx);
-        load_pair(G.pairs + 8 * (size_t)idx[0], k.v[0], k.v[3]);
-        load_pair(G.pairs + 8 * (size_t)idx[1], k.v[1], k.v[4]);
-        load_pair(G.pairs + 8 * (size_t)idx[2], k.v[2], k.v[5]);
-        load_pair(G.pairs + 8 * (size_t)idx[6], k.v[6], k.v[7]);
-    } else {
-        size_t idx[8];
-        corner_indices(G, c.lo, idx);
+    Index idx[8];
+    corner_indices(G, c.lo, idx);
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const float *g = G.g + 3 * idx[q];
-            k.v[q][0] = __ldg(g); k.v[q][1] = __ldg(g + 1); k.v[q][2] = __ldg(g + 2);
-        }
+    for (int q = 0; q < 8; q++) {
+        const float *g = G.g + 3 * idx[q];
+        k.v[q][0] = __ldg(g); k.v[q][1] = __ldg(g + 1); k.v[q][2] = __ldg(g + 2);
     }
 #pragma unroll
     for (int a = 0; a < 3; a++) k.lo[a] = c.lo[a];
@@ -234,11 +200,11 @@ __device__ __forceinline__ Rotation rotate(v3 u0, v3 B, double kappa) {
     return r;
 }
 
-template <bool PAIRS>
+template <class Index>
 __device__ __forceinline__ void step(const AdjGrid &G, Corners &k, v3 &x, v3 &u, double hh, double kappa) {
     const v3 x1 = axpy(u, hh, x);
     const CellPos c = locate(G, x1);
-    load_corners<PAIRS>(G, c, k);
+    load_corners<Index>(G, c, k);
     double w[8];
     weights(c, w);
     const Rotation r = rotate(u, interpolate(k, w), kappa);
@@ -270,7 +236,7 @@ __global__ void kappa_max_kernel(IO io, double h, unsigned long long *kmax) {
 // evenly than 782 blocks of 128.
 constexpr int kForwardBlock = 64, kReverseBlock = 64;
 
-template <bool PAIRS>
+template <class Index>
 __global__ void __launch_bounds__(kForwardBlock, 10) forward_kernel(AdjGrid G, IO io, double h, int n_steps, int K,
                                                                     double *ckpt) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -289,7 +255,7 @@ __global__ void __launch_bounds__(kForwardBlock, 10) forward_kernel(AdjGrid G, I
             c[3 * n + i] = u.x; c[4 * n + i] = u.y; c[5 * n + i] = u.z;
         }
         const int m = n_steps - k0 < every ? n_steps - k0 : every;
-        for (int k = 0; k < m; k++) step<PAIRS>(G, corners, x, u, hh, kappa);
+        for (int k = 0; k < m; k++) step<Index>(G, corners, x, u, hh, kappa);
     }
     io.loss[i] = 1 - dot(u, mk(io.tx[i], io.ty[i], io.tz[i]));
     if (io.ux) { io.ux[i] = u.x; io.uy[i] = u.y; io.uz[i] = u.z; }
@@ -300,11 +266,10 @@ __global__ void __launch_bounds__(kForwardBlock, 10) forward_kernel(AdjGrid G, I
 // stay below 2^50 the rounding is one multiply-add onto 1.5 * 2^52 and the
 // integer its low mantissa bits (24 FP64-to-integer conversions per flush
 // occupied the conversion unit longer than the multiply-adds do).
-template <bool PAIRS>
+template <class Index>
 __device__ __forceinline__ void flush(const AdjGrid &G, unsigned long long *acc, const int lo[3], double g[8][3],
                                       double scale, double &most) {
     if (lo[0] >= 0) {
-        using Index = typename std::conditional<PAIRS, unsigned, size_t>::type;
         Index idx[8];
         corner_indices(G, lo, idx);
         if (most * scale < 1125899906842624.0) {
@@ -332,12 +297,15 @@ __device__ __forceinline__ void flush(const AdjGrid &G, unsigned long long *acc,
 // them FP64) at the warps its registers allow: 6 blocks of 64 (168 registers,
 // of which 72 hold the cell's corners and gradient sums).  Measured over 10^5
 // candidates x 2000 steps, 128^3 grid, checkpoints every 100, forward and
-// reverse kernels with their Python wrapper: 27.3 ms before the corner cache,
-// pair records, Newton reciprocals and FP64-to-integer rounding by addition;
-// 19.2 ms now (forward pass 8.5 -> 3.5 ms); 25.2 ms at 8 blocks (128
-// registers, 656 B of spills), 19.5 ms at 5.
+// reverse kernels with their Python wrapper: 27.0 ms before the corner cache,
+// Newton reciprocals and FP64-to-integer rounding by addition; 19.1 ms now
+// (forward pass 8.5 -> 3.6 ms); 25.2 ms at 8 blocks (128 registers, 656 B of
+// spills), 19.5 ms at 5.  A copy of the grid in pair records (a cell and its upper
+// z neighbour in 32 bytes, four wide loads per cell) gave another 1 % here, but cost
+// 44 B per cell of traffic on every tape: 0.43 -> 1.51 ms for 1000 candidates x 100
+// steps through 512^3 cells.
 constexpr int kReverseMinBlocks = 6;
-template <bool PAIRS>
+template <class Index>
 __global__ void __launch_bounds__(kReverseBlock, kReverseMinBlocks) reverse_kernel(AdjGrid G, IO io, double h,
                                                       int n_steps, int K, const double *ckpt,
                                                       unsigned long long *acc,
@@ -371,7 +339,7 @@ __global__ void __launch_bounds__(kReverseBlock, kReverseMinBlocks) reverse_kern
         // and u: checkpoint_every = 1 recomputes and stores nothing)
         for (int k = 0; k + 1 < m; k++) {
             xs[k] = x; us[k] = u;
-            step<PAIRS>(G, corners, x, u, hh, kappa);
+            step<Index>(G, corners, x, u, hh, kappa);
         }
         for (int k = m - 1; k >= 0; k--) {
             const v3 u0 = u;
@@ -379,11 +347,11 @@ __global__ void __launch_bounds__(kReverseBlock, kReverseMinBlocks) reverse_kern
             // the state before the previous step, asked for a step ahead
             if (k > 0) { x = xs[k - 1]; u = us[k - 1]; }
             if (acc && (cp.lo[0] != glo[0] || cp.lo[1] != glo[1] || cp.lo[2] != glo[2])) {
-                flush<PAIRS>(G, acc, glo, gacc, scale, most);
+                flush<Index>(G, acc, glo, gacc, scale, most);
 #pragma unroll
                 for (int a = 0; a < 3; a++) glo[a] = cp.lo[a];
             }
-            load_corners<PAIRS>(G, cp, corners);
+            load_corners<Index>(G, cp, corners);
             double w[8];
             weights(cp, w);
             const v3 B = interpolate(corners, w);
@@ -429,7 +397,7 @@ __global__ void __launch_bounds__(kReverseBlock, kReverseMinBlocks) reverse_kern
             ub = axpy(xb, hh, ubar);
         }
     }
-    if (acc) flush<PAIRS>(G, acc, glo, gacc, scale, most);
+    if (acc) flush<Index>(G, acc, glo, gacc, scale, most);
     io.gdx[i] = ub.x; io.gdy[i] = ub.y; io.gdz[i] = ub.z;
     io.ge[i] = kb * (-kappa / io.energy[i]);
 }
@@ -480,7 +448,6 @@ AdjGrid make_grid(const crp_adjoint_desc *d) {
     G.goz = d->origin[2] + d->spacing[2] / 2;
     G.sx = d->spacing[0]; G.sy = d->spacing[1]; G.sz = d->spacing[2];
     G.isx = 1.0 / G.sx; G.isy = 1.0 / G.sy; G.isz = 1.0 / G.sz;
-    G.pairs = nullptr;
     return G;
 }
 
@@ -496,6 +463,14 @@ IO make_io(const crp_adjoint_io *a) {
 
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
+bool small_grid(const crp_adjoint_desc *d) { return (size_t)d->nx * d->ny * d->nz <= kSmallGrid; }
+
+void launch_forward(const crp_adjoint_desc *d, const crp_adjoint_io *a, double *ckpt, cudaStream_t s) {
+    auto forward = small_grid(d) ? forward_kernel<unsigned> : forward_kernel<size_t>;
+    forward<<<(unsigned)((a->n + kForwardBlock - 1) / kForwardBlock), kForwardBlock, 0, s>>>(
+        make_grid(d), make_io(a), d->step, d->n_steps, d->checkpoint_every, ckpt);
+}
+
 }  // namespace
 
 extern "C" {
@@ -506,8 +481,7 @@ crp_status crp_bp_adjoint_workspace(const crp_adjoint_desc *d, uint64_t n, size_
         return fail(CRP_ERR_CAPACITY, "checkpoint_every must be 1..128");
     const size_t nck = (size_t)((d->n_steps + d->checkpoint_every - 1) / d->checkpoint_every);
     const size_t cells = (size_t)d->nx * d->ny * d->nz;
-    *bytes = align256(256) + align256(nck * 6 * n * sizeof(double)) + align256(cells * 3 * sizeof(unsigned long long)) +
-             (cells <= kPairCells ? align256(cells * 8 * sizeof(float)) : 0);
+    *bytes = align256(256) + align256(nck * 6 * n * sizeof(double)) + align256(cells * 3 * sizeof(unsigned long long));
     return CRP_OK;
 }
 
@@ -515,8 +489,7 @@ crp_status crp_bp_forward_loss(const crp_adjoint_desc *d, const crp_adjoint_io *
     crp_status st = check_desc(d, a);
     if (st) return st;
     if (a->n == 0) return CRP_OK;
-    forward_kernel<false><<<(unsigned)((a->n + kForwardBlock - 1) / kForwardBlock), kForwardBlock, 0, (cudaStream_t)stream>>>(
-        make_grid(d), make_io(a), d->step, d->n_steps, d->checkpoint_every, nullptr);
+    launch_forward(d, a, nullptr, (cudaStream_t)stream);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CRP_OK : cuda_fail(e, "adjoint forward kernel launch");
 }
@@ -540,11 +513,7 @@ static crp_status adjoint_impl(const crp_adjoint_desc *d, const crp_adjoint_io *
     double *ckpt = reinterpret_cast<double *>(w + align256(256));
     const size_t cells3 = (size_t)d->nx * d->ny * d->nz * 3;
     unsigned long long *acc = reinterpret_cast<unsigned long long *>(w + align256(256) + align256(nck * 6 * a->n * sizeof(double)));
-    AdjGrid G = make_grid(d);
-    const size_t cells = cells3 / 3;
-    // (a workspace off the records' 32-byte alignment reads the grid in place)
-    if (cells <= kPairCells && reinterpret_cast<uintptr_t>(workspace) % 32 == 0)
-        G.pairs = reinterpret_cast<const float *>(reinterpret_cast<char *>(acc) + align256(cells3 * sizeof(unsigned long long)));
+    const AdjGrid G = make_grid(d);
     const IO io = make_io(a);
     auto blocks = [&](unsigned threads) { return (unsigned)((a->n + threads - 1) / threads); };
     cudaError_t e = cudaSuccess;
@@ -552,28 +521,16 @@ static crp_status adjoint_impl(const crp_adjoint_desc *d, const crp_adjoint_io *
         e = cudaMemsetAsync(kmax, 0, 8, s);
         if (e != cudaSuccess) return cuda_fail(e, "clearing the adjoint workspace");
         kappa_max_kernel<<<blocks(128), 128, 0, s>>>(io, d->step, kmax);
-        if (G.pairs) {
-            pair_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(
-                G.g, G.nz, (unsigned)cells, reinterpret_cast<float4 *>(const_cast<float *>(G.pairs)));
-            forward_kernel<true><<<blocks(kForwardBlock), kForwardBlock, 0, s>>>(G, io, d->step, d->n_steps,
-                                                                                 d->checkpoint_every, ckpt);
-        } else {
-            forward_kernel<false><<<blocks(kForwardBlock), kForwardBlock, 0, s>>>(G, io, d->step, d->n_steps,
-                                                                                  d->checkpoint_every, ckpt);
-        }
+        launch_forward(d, a, ckpt, s);
     }
     if (do_backward) {
         if (a->grad_grid) {
             e = cudaMemsetAsync(acc, 0, cells3 * sizeof(unsigned long long), s);
             if (e != cudaSuccess) return cuda_fail(e, "clearing the adjoint workspace");
         }
-        unsigned long long *grad = a->grad_grid ? acc : nullptr;
-        if (G.pairs)
-            reverse_kernel<true><<<blocks(kReverseBlock), kReverseBlock, 0, s>>>(G, io, d->step, d->n_steps,
-                                                                                 d->checkpoint_every, ckpt, grad, kmax);
-        else
-            reverse_kernel<false><<<blocks(kReverseBlock), kReverseBlock, 0, s>>>(G, io, d->step, d->n_steps,
-                                                                                  d->checkpoint_every, ckpt, grad, kmax);
+        auto reverse = small_grid(d) ? reverse_kernel<unsigned> : reverse_kernel<size_t>;
+        reverse<<<blocks(kReverseBlock), kReverseBlock, 0, s>>>(G, io, d->step, d->n_steps, d->checkpoint_every, ckpt,
+                                                                a->grad_grid ? acc : nullptr, kmax);
         if (a->grad_grid)
             finalize_kernel<<<(unsigned)((cells3 + 255) / 256), 256, 0, s>>>(acc, cells3, kmax, a->grad_grid);
     }

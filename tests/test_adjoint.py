@@ -169,3 +169,47 @@ def test_adjoint_in_a_workspace_of_any_alignment():
         got.append([a.cpu().numpy() for a in (loss, *gu, ge, gg)])
     for a, b in zip(*got):
         np.testing.assert_array_equal(a, b)
+
+
+def test_adjoint_workspace_holds_checkpoints_and_sums_only():
+    """48 bytes per candidate and checkpoint, 24 per cell: no copy of the grid, however few
+    steps the candidates make through however large a one."""
+    import ctypes as C
+    from crpropa3_b200 import _abi
+    from crpropa3_b200.adjoint import _desc
+
+    class Grid:
+        shape = (512, 256, 257, 3)
+
+        def data_ptr(self):
+            return 0
+
+    d, need = _desc(Grid(), ORIGIN, SPACING, STEP, 50, 10), C.c_size_t()
+    _abi.check(_abi.load().crp_bp_adjoint_workspace(C.byref(d), 1000, C.byref(need)))
+    assert need.value <= 48 * 1000 * 5 + 24 * 512 * 256 * 257 + 3 * 256
+
+
+def test_adjoint_tape_may_move():
+    """The reverse pass reads checkpoints and the grid, wherever the workspace's copy lies."""
+    import ctypes as C
+    import torch
+    from crpropa3_b200 import _abi
+    from crpropa3_b200.adjoint import _desc, _io, _planar
+    grid, pos, u0, energy, charge, target = _problem(n=40, seed=87)
+    want = _gpu(grid, pos, u0, energy, charge, target)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    g, lib = t(grid), _abi.load()
+    d, need = _desc(g, ORIGIN, SPACING, STEP, NSTEPS, K), C.c_size_t()
+    _abi.check(lib.crp_bp_adjoint_workspace(C.byref(d), 40, C.byref(need)))
+    ins = [_planar(t(a)) for a in (pos, u0, target)]
+    E = lambda *s: torch.zeros(*s, dtype=torch.float64, device="cuda")
+    loss, ge, gu, gg = E(40), E(40), [E(40) for _ in range(3)], E(*g.shape)
+    io = _io(40, ins[0], ins[1], t(energy), t(charge), ins[2], loss, None, gu, ge, gg)
+    keep = t(energy), t(charge)
+    io.energy, io.charge = keep[0].data_ptr(), keep[1].data_ptr()
+    a, b = torch.zeros(need.value + 8, dtype=torch.uint8, device="cuda"), torch.zeros(need.value, dtype=torch.uint8, device="cuda")
+    _abi.check(lib.crp_bp_adjoint_forward(C.byref(d), C.byref(io), C.c_void_p(a.data_ptr() + 8), need.value, None))
+    b.copy_(a[8:])
+    _abi.check(lib.crp_bp_adjoint_backward(C.byref(d), C.byref(io), C.c_void_p(b.data_ptr()), need.value, None))
+    for got, ref in zip((loss, torch.stack(gu, 1), ge, gg), want):
+        np.testing.assert_array_equal(got.cpu().numpy(), ref)
