@@ -262,9 +262,10 @@ crp_status build_grid(crp_plan *p, const crp_grid3f_desc &g, int comps, DevGrid 
         return fail(CRP_ERR_INVALID_ARGUMENT, "%s: interpolation type not understood", name);
     const size_t cells = (size_t)g.nx * g.ny * g.nz;
     dg.pairs = nullptr;
-    // records and values in one allocation
+    // records (for the trilinear gathers that read them) and values in one allocation
     void *d = nullptr;
-    const size_t records = comps == 3 && cells <= kPairCells ? cells * 32 : 0;
+    const size_t records =
+        comps == 3 && cells <= kPairCells && g.interpolation == CRP_INTERPOLATION_TRILINEAR ? cells * 32 : 0;
     cudaError_t e = records ? cudaMalloc(&d, records + cells * 12) : cudaErrorMemoryAllocation;
     if (e == cudaSuccess) {
         p->owned.push_back(d);
