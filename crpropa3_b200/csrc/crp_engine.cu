@@ -721,11 +721,12 @@ crp_status crp_plan_create(const crp_plan_desc *desc, crp_plan **out) {
         }
     }
     if (d.n_fields == 1 && !desc->fields[0].periodic && desc->fields[0].kind == CRP_FIELD_GRID) {
-        const DevGrid &g = d.fields[0].grid;
-        const bool small = g.pairs != nullptr;  // at most 2^30 cells: 32-bit cell indices
+        DevGrid &g = d.fields[0].grid;
+        const bool small = (uint64_t)g.nx * g.ny * g.nz < (1ull << 31);  // 32-bit cell indices
         const bool trilinear = g.interp == CRP_INTERPOLATION_TRILINEAR;
-        p->fs = (!g.reflective && !g.clip_volume && g.pow2 && small && trilinear) ? FS_GRID_PERIODIC
-                                                                                           : FS_GRID;
+        // whether the pair records found room decides the kernel, not the result
+        g.rounded = !g.reflective && !g.clip_volume && g.pow2 && small && trilinear;
+        p->fs = g.rounded && g.pairs ? FS_GRID_PERIODIC : FS_GRID;
     }
     else if (d.n_fields == 1 && !desc->fields[0].periodic && desc->fields[0].kind == CRP_FIELD_PLANE_WAVE)
         p->fs = FS_PLANE_WAVE;

@@ -29,7 +29,8 @@ struct DevGrid {
     double ox, oy, oz;     // origin (clipVolume test)
     double ex, ey, ez;     // origin + N*spacing (clipVolume test, Grid.h:322)
     int interp;            // crp_interpolation
-    int pad_;
+    int rounded;           // mixed fixed-step Boris push: cell fractions from the rounded coordinates, as
+                           // FS_GRID_PERIODIC kernels form them (grid_field_t)
 };
 
 // What cos_turns (mixed_device.cuh) adds to a mode's fixed-point phase: half a

@@ -125,7 +125,8 @@ __device__ __forceinline__ f3 grid_cell_interp(const CellFrac &f, const float (&
 
 // FUSED: the cell fraction from the unrounded product of position and inverse
 // spacing (one multiply-add), as the fixed-step Boris kernels over any grid
-// form it; otherwise from the rounded coordinate.  Written out so that it does
+// form it; otherwise, and for grids marked `rounded` (FS_GRID_PERIODIC's, where
+// their pair records found no room), from the rounded coordinate.  Written out so that it does
 // not depend on how the compiler contracts the expression in each kernel.
 template <bool CACHE, bool PER = false, bool FUSED = false>
 __device__ __forceinline__ f3 grid_field_t(const DevGrid &g, double x, double y, double z, Cand *cc) {
@@ -144,7 +145,7 @@ __device__ __forceinline__ f3 grid_field_t(const DevGrid &g, double x, double y,
     double rx = (x - g.gox) * g.inv_sx, ry = (y - g.goy) * g.inv_sy, rz = (z - g.goz) * g.inv_sz;
     double flx = floor(rx), fly = floor(ry), flz = floor(rz);
     float fx0, fy0, fz0;
-    if (FUSED) {
+    if (FUSED && !g.rounded) {
         fx0 = (float)fma(x - g.gox, g.inv_sx, -flx);
         fy0 = (float)fma(y - g.goy, g.inv_sy, -fly);
         fz0 = (float)fma(z - g.goz, g.inv_sz, -flz);

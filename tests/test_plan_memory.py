@@ -31,3 +31,37 @@ def _plan_and_bytes(spec):
 def test_grids_that_no_kernel_gathers_in_pairs_hold_their_values_only(precision, interpolation):
     _, used = _plan_and_bytes(_spec(precision, interpolation))
     assert 12 * CELLS <= used <= 12 * CELLS + (8 << 20)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [_abi.PRECISION_FP64, _abi.PRECISION_MIXED])
+@pytest.mark.parametrize("n_extra", [0, 1, 2])
+def test_same_results_where_the_pair_records_find_no_room(precision, n_extra):
+    """[fixed BP, MaximumTrajectoryLength], with an observer and with two, over a periodic
+    power-of-two grid: free memory decides the kernel, never the trajectories."""
+    import torch
+    from crpropa3_b200.engine import Plan
+    rng = np.random.default_rng(3)
+    values = (rng.standard_normal(SHAPE + (3,)) * 3e-13).astype(np.float32)
+    extra = [P.ObserverSpec(features=[P.Feature(_abi.OBSERVER_PARTICLE_ID_VETO, particle_id=77)])] * n_extra
+    spec = _spec(precision, values=values, extra=extra)
+    c = protons(rng, 500, emin=0.1 * U.EeV, spread=1e7 * U.kpc)  # fractions of coordinates near 10^6
+    small = _spec(precision, values=np.zeros((5, 3, 2, 3), np.float32), extra=extra)
+    Plan(small).run(c.copy())  # the general grid's kernel, loaded while there is room for it
+    want, got = c.copy(), c.copy()
+    plan = Plan(spec)
+    plan.run(want)
+    del plan
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    room = 12 * CELLS + 32 * CELLS - (64 << 20)  # for the values, not for their records beside them
+    fill = torch.empty(free - room, dtype=torch.uint8, device="cuda")
+    try:
+        plan, used = _plan_and_bytes(spec)
+        plan.run(got)
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert used < 16 * CELLS
+    for name, a in want.members().items():
+        np.testing.assert_array_equal(getattr(got, name), a, err_msg=name)
