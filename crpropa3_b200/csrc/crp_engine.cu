@@ -741,6 +741,7 @@ crp_status crp_plan_create(const crp_plan_desc *desc, crp_plan **out) {
     if (st) { delete p; return st; }
     if (cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device) != cudaSuccess)
         p->num_sms = 148;
+    d.num_sms = p->num_sms;
     *out = p;
     return CRP_OK;
 }

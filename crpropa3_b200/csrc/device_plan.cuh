@@ -179,6 +179,7 @@ struct DevPlan {
     int n_modules;
     int prop_index;  // position of the propagation module in the chain
     int shape;       // ChainShape (chain.cuh) the module sequence matches
+    int num_sms;     // of the plan's device
     int block_warps; // FS_PLANE_WAVE_BLOCK: warps of a block that hold candidates (set per launch)
     uint64_t seed;
     DevComponent fields[kMaxFields];

@@ -55,21 +55,53 @@ inline int lanes_per_warp(uint64_t n, int num_sms, int warps_per_sm) {
 // Runs up to this size ask for the next grid cell ahead (step_*_bp.cu).
 constexpr uint64_t kAskAheadCandidates = 592 * 40;
 
-// Warps of candidates per block of a chunked launch over a PlaneWaveTurbulence
-// field evaluated by the block: the fewest whose blocks are resident at once (592:
-// four per SM), so that a small run has the most warps per candidate.  0: each
-// thread sums for itself, for fewer modes than pay for the barriers, for tables
-// that leave room for one block per SM only, and in the FP64 form for runs that
-// fill the GPU thread by thread (its terms are added by three warps of four:
-// 10^5 candidates, 100 modes: 1.50 ms thread by thread, 2.07 ms by blocks;
-// 20 000 candidates, 200 modes: 5.16 and 4.06 ms; the mixed form 4 x 10^5
-// candidates, 300 modes: 7.08 and 3.92 ms, 20 modes: 0.86 and 0.82 ms).
+// Chunked launches over a PlaneWaveTurbulence field summed by the block
+// (FS_PLANE_WAVE_BLOCK).  The largest table taken: 98 KB in the FP64 form, two blocks
+// per SM beside the kernel's own 11 KB.
 constexpr int kWaveMaxModes = 1365;
-inline int wave_block_warps(uint64_t n, int n_modes, bool fp64) {
+// Blocks per SM that the kernels' registers are held to.  FP64 Cash-Karp spills 300 B
+// at 4 (14 000 candidates x 200 modes: 1.45 ms, 1.23 at 3); the FP64 push loses at 3.
+// The mixed adaptive push is faster at 3 below 37 888 candidates (3000 x 200 modes:
+// 0.177 and 0.117 ms) and slower above (75 000: 0.48 and 0.50).
+constexpr int wave_blocks(bool fp64, bool ck) { return fp64 && ck ? 3 : 4; }
+// Blocks per SM of one launch: those, or as many as fit in 228 KB of shared memory
+// (the table, the kernel's own arrays and 1 KB of the system's each).
+inline uint64_t wave_blocks_per_sm(int n_modes, bool fp64, bool ck) {
+    const size_t block = (fp64 ? 11 * 1024 + (size_t)n_modes * 72 : 9 * 1024 + (size_t)((n_modes + 1) / 2) * 80) + 1024;
+    const uint64_t room = 228 * 1024 / block, most = (uint64_t)wave_blocks(fp64, ck);
+    return room < most ? room : most;
+}
+
+// Warps of candidates per block of such a launch; 0: each thread sums for itself.
+// A block of four warps sums the modes for 32 candidates (or 64, 128: fewer
+// blocks, more candidates per table read).
+//
+// FP64 (its terms are added by three warps of four): the sums by the block pay
+// while all blocks are resident at once, else a run that fills the GPU thread by
+// thread is faster (fixed push: 18 900 candidates x 500 modes 1.05 ms with
+// blocks left over, 0.93 thread by thread, 0.73 by 64; 28 000 x 1000 modes 2.82
+// and 1.94 ms).  64 per block at four blocks per SM pay for long sums only (37 800
+// candidates: 40 modes 1.07, 100 modes 0.94 of the time thread by thread).
+//
+// Mixed: 32 while those blocks are resident at once, then 64, then 128 (fixed push,
+// 4 x 10^5 candidates x 300 modes: 7.08 ms thread by thread, 3.92 here).  Cash-Karp
+// holds its stages meanwhile, and more candidates per block wait longer: sums of
+// 100 modes stay at 32 per block up to 20 blocks per SM, of 200 always (28 000 x 200
+// modes: 0.26 ms, 0.41 at 64, 0.45 thread by thread; 150 000 x 100: 0.89, 0.82 at
+// 128).  Where two full warps per scheduler sum for themselves, that is the faster
+// up to 500 modes (37 800 x 100 modes: 0.25 ms, 0.29 at 32, 0.32 at 64; x 500: 1.06
+// and 0.98).
+inline int wave_block_warps(uint64_t n, int n_modes, int num_sms, bool fp64, bool ck) {
     if (n_modes < (fp64 ? 32 : 8) || n_modes > kWaveMaxModes) return 0;
-    if (n <= 592u * 32u) return 1;
-    if (n <= 592u * 64u) return 2;
-    return fp64 ? 0 : 4;
+    const uint64_t sms = (uint64_t)num_sms, per_sm = wave_blocks_per_sm(n_modes, fp64, ck);
+    auto blocks = [n](int warps) { return (n + 32 * (uint64_t)warps - 1) / (32 * (uint64_t)warps); };
+    if (blocks(1) <= per_sm * sms) return 1;
+    if (fp64) return blocks(2) <= (per_sm == 4 && n_modes < 100 ? 3 : per_sm) * sms ? 2 : 0;
+    if (ck) {
+        if (n_modes < 500 && blocks(1) > 6 * sms && blocks(1) <= 8 * sms) return 0;
+        if (n_modes >= 200 || (n_modes >= 100 && blocks(1) <= 20 * sms)) return 1;
+    }
+    return blocks(2) <= 4 * sms ? 2 : 4;
 }
 
 // Dynamic shared memory a kernel may be launched with: MOST, the largest that

@@ -292,12 +292,12 @@ __device__ d3 plane_wave_field(const DevPlaneWave &w, d3 pos) {
 
 // The same sum for a block's candidates (FS_PLANE_WAVE_BLOCK kernels; every
 // thread of the block calls it): the sum over the modes is one chain in the
-// reference's order, but its terms are not.  The block's first 32 wp threads hold
-// the candidates; per round of kWaveRound modes the four warps evaluate the
-// cosines of a quarter of the modes each for all of them, and warp a < 3 adds
+// reference's order, but its terms are not.  The block's first 32 wp threads (wp 1 or
+// 2) hold the candidates; per round of kWaveRound modes the four warps evaluate
+// the cosines of a quarter of the modes each for all of them, and warp a < 3 adds
 // component a of the round's terms in order.  3001 candidates x 60 steps x 77
 // modes: 1.32 ms thread by thread, 0.83 ms here.
-constexpr int kBatchThreads = 128, kWaveRound = 16;
+constexpr int kBatchThreads = 128, kWaveRound = 16, kWaveCandidates = 64;
 inline size_t wave_table_bytes(const DevPlaneWave &w) { return (size_t)w.n * 72; }
 __device__ __forceinline__ void stage_wave_table(const DevPlaneWave &w, unsigned char *to) {
     double *t = reinterpret_cast<double *>(to);
@@ -305,12 +305,13 @@ __device__ __forceinline__ void stage_wave_table(const DevPlaneWave &w, unsigned
 }
 
 __device__ __forceinline__ d3 plane_wave_block(const DevPlaneWave &w, d3 pos, int wp) {
-    __shared__ double qpos[3][kBatchThreads], cosine[kWaveRound][kBatchThreads], sum[3][kBatchThreads];
+    __shared__ double qpos[3][kWaveCandidates], cosine[kWaveRound][kWaveCandidates], sum[3][kWaveCandidates];
     extern __shared__ __align__(16) unsigned char pw_table[];
     const double *tab = reinterpret_cast<const double *>(pw_table);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    qpos[0][t] = pos.x; qpos[1][t] = pos.y; qpos[2][t] = pos.z;
-    double acc[4] = {0, 0, 0, 0};  // of candidates lane + 32 j, component `warp`
+    const int mine = t < kWaveCandidates ? t : 0;  // threads past the candidates take any sum
+    if (t < kWaveCandidates) { qpos[0][t] = pos.x; qpos[1][t] = pos.y; qpos[2][t] = pos.z; }
+    double acc[2] = {0, 0};  // of candidates lane + 32 j, component `warp`
     for (int m0 = 0; m0 < w.n; m0 += kWaveRound) {
         const int m1 = min(w.n - m0, kWaveRound);
         __syncthreads();
@@ -329,15 +330,15 @@ __device__ __forceinline__ d3 plane_wave_block(const DevPlaneWave &w, d3 pos, in
                 const double *q = tab + 9 * (m0 + m);
                 const double a = q[warp] * q[8];
 #pragma unroll
-                for (int j = 0; j < 4; j++)
+                for (int j = 0; j < 2; j++)
                     if (j < wp) acc[j] = acc[j] + a * cosine[m][lane + 32 * j];
             }
     }
 #pragma unroll
-    for (int j = 0; j < 4; j++)
+    for (int j = 0; j < 2; j++)
         if (warp < 3 && j < wp) sum[warp][lane + 32 * j] = acc[j];
     __syncthreads();
-    return mk(sum[0][t], sum[1][t], sum[2][t]);
+    return mk(sum[0][mine], sum[1][mine], sum[2][mine]);
 }
 
 // ---------------------------------------------------------------- JF12Field
@@ -551,6 +552,7 @@ __device__ __forceinline__ void set_direction(Cand &c, d3 uo) {
 template <int FS, int MODE = 0>
 struct BP {
     static constexpr bool kReadsStepCount = false;
+    static constexpr bool kCashKarp = false;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
     static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
     // PropagationBP::process (PropagationBP.cpp:62): its start (false when the
@@ -678,6 +680,7 @@ __device__ __forceinline__ void ck_try(const DevPlan &P, d3 x, d3 u, double h, d
 template <int FS, int MODE = 0>
 struct CK {
     static constexpr bool kReadsStepCount = false;
+    static constexpr bool kCashKarp = true;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
     static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
     // PropagationCK::process (PropagationCK.cpp:77): its start (false when the
@@ -932,7 +935,7 @@ fp64_boris_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, int
 
 // Kernels of FS_PLANE_WAVE_BLOCK: the mode table staged in dynamic shared memory.
 template <template <int> class Prop, int CS>
-__global__ void __launch_bounds__(kBatchThreads, 4)
+__global__ void __launch_bounds__(kBatchThreads, wave_blocks(true, Prop<FS_PLANE_WAVE_BLOCK>::kCashKarp))
 fp64_wave_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, int max_steps, uint64_t step_cap,
                   DevCounters *cnt, DevRecords rec, const uint32_t *perm, uint32_t *perm_out) {
     extern __shared__ __align__(16) unsigned char pw_table[];
@@ -965,7 +968,9 @@ cudaError_t launch_prop(const DevPlan &P, const DevState &s, uint64_t n, int max
                         const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
                         cudaStream_t st) {
     if constexpr (Prop<FS_PLANE_WAVE>::kBlockField) {
-        const int warps = fs == FS_PLANE_WAVE ? wave_block_warps(n, P.fields[0].pw.n, true) : 0;
+        const int warps =
+            fs == FS_PLANE_WAVE
+                ? wave_block_warps(n, P.fields[0].pw.n, P.num_sms, true, Prop<FS_PLANE_WAVE>::kCashKarp) : 0;
         if (warps) return launch_waves<Prop>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, warps, st);
     }
     const uint64_t slots = (uint64_t)(block / 32) * (uint64_t)lanes;

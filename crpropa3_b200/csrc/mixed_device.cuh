@@ -1185,6 +1185,7 @@ __device__ __forceinline__ void bp_dy(const DevPlan &P, double &x, double &y, do
 template <int FS, int MODE = 0>
 struct BP {
     static constexpr bool kReadsStepCount = false;
+    static constexpr bool kCashKarp = false;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
     static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
     struct Try {
@@ -1330,6 +1331,7 @@ __device__ __forceinline__ double ck_try(const DevPlan &P, Cand &c, double h, fl
 template <int FS, int MODE = 0>
 struct CK {
     static constexpr bool kReadsStepCount = false;
+    static constexpr bool kCashKarp = true;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
     static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
     struct Try {
@@ -1693,7 +1695,7 @@ mixed_boris_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, in
 
 // Kernels of FS_PLANE_WAVE_BLOCK: the mode table staged in dynamic shared memory.
 template <template <int> class Prop, int CS>
-__global__ void __launch_bounds__(kBatchThreads, 4)
+__global__ void __launch_bounds__(kBatchThreads, wave_blocks(false, Prop<FS_PLANE_WAVE_BLOCK>::kCashKarp))
 mixed_wave_kernel(const __grid_constant__ DevPlan P, DevState s, uint64_t n, int max_steps, uint64_t step_cap,
                   DevCounters *cnt, DevRecords rec, const uint32_t *perm, uint32_t *perm_out) {
     extern __shared__ __align__(16) unsigned char pw_table[];
@@ -1726,7 +1728,9 @@ cudaError_t launch_prop(const DevPlan &P, const DevState &s, uint64_t n, int max
                         const uint32_t *perm, uint32_t *perm_out, int fs, int block, int lanes,
                         cudaStream_t st) {
     if constexpr (Prop<FS_PLANE_WAVE>::kBlockField) {
-        const int warps = fs == FS_PLANE_WAVE ? wave_block_warps(n, P.fields[0].pw.n, false) : 0;
+        const int warps =
+            fs == FS_PLANE_WAVE
+                ? wave_block_warps(n, P.fields[0].pw.n, P.num_sms, false, Prop<FS_PLANE_WAVE>::kCashKarp) : 0;
         if (warps) return launch_waves<Prop>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, warps, st);
     }
     const uint64_t slots = (uint64_t)(block / 32) * (uint64_t)lanes;
