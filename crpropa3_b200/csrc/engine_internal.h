@@ -88,17 +88,18 @@ inline uint64_t wave_blocks_per_sm(int n_modes, bool fp64, bool ck) {
 // holds its stages meanwhile, and more candidates per block wait longer: sums of
 // 100 modes stay at 32 per block up to 20 blocks per SM, of 200 always (28 000 x 200
 // modes: 0.26 ms, 0.41 at 64, 0.45 thread by thread; 150 000 x 100: 0.89, 0.82 at
-// 128).  Where two full warps per scheduler sum for themselves, that is the faster
-// up to 500 modes (37 800 x 100 modes: 0.25 ms, 0.29 at 32, 0.32 at 64; x 500: 1.06
-// and 0.98).
-inline int wave_block_warps(uint64_t n, int n_modes, int num_sms, bool fp64, bool ck) {
+// 128).  Where two full warps per scheduler sum for themselves and no observer or
+// boundary divides them (pm: the chain ends with MaximumTrajectoryLength), that is
+// the faster up to 500 modes (37 800 x 100 modes: 0.25 ms, 0.29 at 32, 0.32 at 64; x
+// 500: 1.06 and 0.98; with an observer 37 000 x 40 modes: 1.04 and 0.80 at 64).
+inline int wave_block_warps(uint64_t n, int n_modes, int num_sms, bool fp64, bool ck, bool pm) {
     if (n_modes < (fp64 ? 32 : 8) || n_modes > kWaveMaxModes) return 0;
     const uint64_t sms = (uint64_t)num_sms, per_sm = wave_blocks_per_sm(n_modes, fp64, ck);
     auto blocks = [n](int warps) { return (n + 32 * (uint64_t)warps - 1) / (32 * (uint64_t)warps); };
     if (blocks(1) <= per_sm * sms) return 1;
     if (fp64) return blocks(2) <= (per_sm == 4 && n_modes < 100 ? 3 : per_sm) * sms ? 2 : 0;
     if (ck) {
-        if (n_modes < 500 && blocks(1) > 6 * sms && blocks(1) <= 8 * sms) return 0;
+        if (pm && n_modes < 500 && blocks(1) > 6 * sms && blocks(1) <= 8 * sms) return 0;
         if (n_modes >= 200 || (n_modes >= 100 && blocks(1) <= 20 * sms)) return 1;
     }
     return blocks(2) <= 4 * sms ? 2 : 4;

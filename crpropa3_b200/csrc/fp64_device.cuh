@@ -970,7 +970,8 @@ cudaError_t launch_prop(const DevPlan &P, const DevState &s, uint64_t n, int max
     if constexpr (Prop<FS_PLANE_WAVE>::kBlockField) {
         const int warps =
             fs == FS_PLANE_WAVE
-                ? wave_block_warps(n, P.fields[0].pw.n, P.num_sms, true, Prop<FS_PLANE_WAVE>::kCashKarp) : 0;
+                ? wave_block_warps(n, P.fields[0].pw.n, P.num_sms, true, Prop<FS_PLANE_WAVE>::kCashKarp, P.shape == CS_PM)
+                : 0;
         if (warps) return launch_waves<Prop>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, warps, st);
     }
     const uint64_t slots = (uint64_t)(block / 32) * (uint64_t)lanes;

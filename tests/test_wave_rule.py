@@ -18,7 +18,7 @@ int main() {
             for (int ck = 0; ck < 2; ck++)
                 for (int m = 1; m <= 1400; m += m < 70 ? 1 : 7)
                     for (uint64_t n = 1; n < 400000; n += 1 + n / 23) {
-                        const int w = crp::wave_block_warps(n, m, sms, fp64, ck);
+                        const int w = crp::wave_block_warps(n, m, sms, fp64, ck, n % 2);
                         const uint64_t blocks = w ? (n + 32 * w - 1) / (32 * w) : 0;
                         const size_t table = fp64 ? 72 * (size_t)m : 80 * (size_t)((m + 1) / 2);
                         const size_t block = table + (fp64 ? 11264 : 9216) + 1024;
