@@ -450,17 +450,17 @@ __device__ d3 component_field(const DevComponent &f, d3 position) {
     }
 }
 
-// MagneticFieldList::getField (MagneticField.cpp:64) or the single field.  Not
-// inlined: the Cash-Karp step evaluates the field six times, and the body of
-// every field class at each is more code than the instruction cache holds.
-// The components are read from device memory (uniform addresses, L1 hits).
-__device__ __noinline__ d3 field_sum(const DevComponent *f, int n, d3 pos) {
+// MagneticFieldList::getField (MagneticField.cpp:64) or the single field.
+__device__ __forceinline__ d3 field_sum(const DevComponent *f, int n, d3 pos) {
     if (n == 1) return component_field(f[0], pos);
     d3 b = mk(0, 0, 0);
 #pragma unroll 1
     for (int i = 0; i < n; i++) b = add(b, component_field(f[i], pos));
     return b;
 }
+// The same as a call (why and where: field_sum_call in mixed_device.cuh; here also in
+// DiffusionSDE, 30 000 pseudo-particles in a toroidal field 0.23 ms inlined, 0.18).
+__device__ __noinline__ d3 field_sum_call(const DevComponent *f, int n, d3 pos) { return field_sum(f, n, pos); }
 
 // A single galactic field, without the sum's tests and loads.
 __device__ __forceinline__ d3 galactic_field(const DevComponent &f, d3 pos) {
@@ -475,14 +475,14 @@ __device__ __forceinline__ d3 galactic_field(const DevComponent &f, d3 pos) {
     return mk(b.x, b.y, b.z);
 }
 
-template <int FS>
+template <int FS, bool CALL = false>
 __device__ __forceinline__ d3 field_at(const DevPlan &P, d3 pos, Cand *cc = nullptr) {
     if (FS == FS_GRID) return grid_field_t<true>(P.fields[0].grid, pos, cc);
     if (FS == FS_GRID_PERIODIC) return grid_field_t<true, true>(P.fields[0].grid, pos, cc);
     if (FS == FS_PLANE_WAVE) return plane_wave_field(P.fields[0].pw, pos);
     if (FS == FS_PLANE_WAVE_BLOCK) return plane_wave_block(P.fields[0].pw, pos, P.block_warps);
     if (FS == FS_GALACTIC) return galactic_field(P.fields[0], pos);
-    return field_sum(P.dev_fields, P.n_fields, pos);
+    return CALL ? field_sum_call(P.dev_fields, P.n_fields, pos) : field_sum(P.fields, P.n_fields, pos);
 }
 
 __device__ __forceinline__ void set_current_step(Cand &c, double s) {  // Candidate.cpp:92
@@ -549,12 +549,12 @@ __device__ __forceinline__ void set_direction(Cand &c, d3 uo) {
     c.dx = u.x; c.dy = u.y; c.dz = u.z;
 }
 
-template <int FS, int MODE = 0>
+template <int FS, int MODE>
 struct BP {
     static constexpr bool kReadsStepCount = false;
     static constexpr bool kCashKarp = false;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
-    static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
+    static constexpr bool kTogether = MODE != 1;  // advance()
     // PropagationBP::process (PropagationBP.cpp:62): its start (false when the
     // step is done, neutral candidates) and one try (true when it is done; threads
     // that only take part in its field evaluations pass on = false).
@@ -650,7 +650,7 @@ __constant__ double ck_b[6] = {37. / 378., 0, 250. / 621., 125. / 594., 0., 512.
 __constant__ double ck_bs[6] = {2825. / 27648., 0., 18575. / 48384., 13525. / 55296.,
                                 277. / 14336., 1. / 4.};
 
-template <int FS>
+template <int FS, bool CALL>
 __device__ __forceinline__ void ck_try(const DevPlan &P, d3 x, d3 u, double h, double q, double E,
                                        d3 &xo, d3 &uo, d3 &eu, Cand *cc) {
     d3 kx[6], ku[6];
@@ -666,7 +666,7 @@ __device__ __forceinline__ void ck_try(const DevPlan &P, d3 x, d3 u, double h, d
             yu = add(yu, muls(muls(ku[j], ck_a[i * 6 + j]), h));
         }
         d3 vel = muls(unit_fast(yu), kCLight);
-        d3 B = field_at<FS>(P, yx, cc);
+        d3 B = field_at<FS, CALL>(P, yx, cc);
         d3 dudt = muls(cross(vel, B), qcE);
         kx[i] = vel; ku[i] = dudt;
         if (i != 1 && i != 4) {  // b_1 = b_4 = 0
@@ -677,12 +677,12 @@ __device__ __forceinline__ void ck_try(const DevPlan &P, d3 x, d3 u, double h, d
     }
 }
 
-template <int FS, int MODE = 0>
+template <int FS, int MODE, bool CALLED>
 struct CK {
     static constexpr bool kReadsStepCount = false;
     static constexpr bool kCashKarp = true;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
-    static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
+    static constexpr bool kTogether = MODE != 1 || FS == FS_GENERIC;  // advance()
     // PropagationCK::process (PropagationCK.cpp:77): its start (false when the
     // step is done, neutral candidates) and one try (true when it is done; threads
     // that only take part in its field evaluations pass on = false).
@@ -704,7 +704,7 @@ struct CK {
                                                    StepCount &sc, bool on = true) {
         double step = t.step, newStep = step;
         d3 xo, uo, eu;
-        ck_try<FS>(P, mk(c.x, c.y, c.z), mk(c.dx, c.dy, c.dz), step / kCLight, c.q, c.E, xo, uo, eu, &c);
+        ck_try<FS, CALLED>(P, mk(c.x, c.y, c.z), mk(c.dx, c.dy, c.dz), step / kCLight, c.q, c.E, xo, uo, eu, &c);
         if (!on) return false;
         sc.tries++; sc.evals += 6;
         if (MODE != 1) {
@@ -758,7 +758,7 @@ __device__ __forceinline__ void sde_try(const DevPlan &P, d3 PosIn, d3 &POut, d3
         d3 y_n = PosIn;
 #pragma unroll
         for (int j = 0; j < i; j++) y_n = add(y_n, muls(muls(k[j], ck_a[i * 6 + j]), propStep));
-        d3 B = field_at<FS>(P, y_n, cc);
+        d3 B = field_at<FS, true>(P, y_n, cc);
         k[i] = muls(unit(B), kCLight);
         POut = add(POut, muls(muls(k[i], ck_b[i]), propStep));
         PosErr = add(PosErr, divs(muls(muls(k[i], ck_b[i] - ck_bs[i]), propStep), CRP_KPC));
@@ -769,7 +769,7 @@ template <int FS>
 struct SDE {
     static constexpr bool kReadsStepCount = true;  // the Philox counter
     static constexpr bool kBlockField = false;
-    static constexpr bool kRetries = false;
+    static constexpr bool kTogether = false;  // advance()
     struct Try {};
     __device__ __forceinline__ static bool begin(const DevPlan &, const DevModule &, Cand &, Try &) { return true; }
     __device__ __forceinline__ static bool attempt(const DevPlan &P, const DevModule &m, Cand &c, Try &,
@@ -866,10 +866,13 @@ template <class T> struct MinBlocks { static constexpr int value = 1; };
 template <int FS, int MODE> struct MinBlocks<BP<FS, MODE>> {
     static constexpr int value = MODE != 1 ? CRP_BP_ADAPTIVE_MIN_BLOCKS : FS == FS_GRID ? CRP_BP_GRID_MIN_BLOCKS : CRP_BP_FIXED_MIN_BLOCKS;
 };
-template <int FS, int MODE> struct MinBlocks<CK<FS, MODE>> { static constexpr int value = CRP_CK_MIN_BLOCKS; };
+template <int FS, int MODE, bool CALLED> struct MinBlocks<CK<FS, MODE, CALLED>> {
+    static constexpr int value = CRP_CK_MIN_BLOCKS;
+};
 template <int FS> using BPAdaptive = BP<FS, 2>;
-template <int FS> using CKFixed = CK<FS, 1>;
-template <int FS> using CKAdaptive = CK<FS, 2>;
+template <int FS> using CKFixed = CK<FS, 1, FS == FS_GENERIC>;
+template <int FS> using CKFixedInlined = CK<FS, 1, false>;  // lists of fields, warps full (step_*_ck.cu)
+template <int FS> using CKAdaptive = CK<FS, 2, FS == FS_GENERIC>;
 
 template <template <int> class Prop, int FS, int CS>
 __global__ void __launch_bounds__(128, MinBlocks<Prop<FS>>::value)

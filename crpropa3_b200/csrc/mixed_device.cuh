@@ -1082,14 +1082,10 @@ __device__ __forceinline__ f3 component_field(const DevComponent &f, double x, d
     }
 }
 
-// The field of any list of components.  Not inlined: the Cash-Karp step
-// evaluates the field six times and the adaptive Boris push three times, and
-// with the body of every field class inlined at each the kernels waited for
-// instructions (no_instruction 1.4-1.6 cycles per issued one).
+// The field of any list of components.
 // sh: the plan's plane-wave table staged in shared memory (at most one
 // plane-wave component), or null.
-// The components are read from device memory (uniform addresses, L1 hits).
-__device__ __noinline__ f3 field_sum(const DevComponent *f, int n, double x, double y, double z, const PwTab *sh) {
+__device__ __forceinline__ f3 field_sum(const DevComponent *f, int n, double x, double y, double z, const PwTab *sh) {
     if (n == 1) return component_field(f[0], x, y, z, sh);
     f3 b = f3mk(0.f, 0.f, 0.f);
 #pragma unroll 1
@@ -1098,6 +1094,20 @@ __device__ __noinline__ f3 field_sum(const DevComponent *f, int n, double x, dou
         b.x += c.x; b.y += c.y; b.z += c.z;
     }
     return b;
+}
+// The same as a call, for Cash-Karp steps: they evaluate the field six times, and
+// with the body of every field class inlined at each the kernels waited for
+// instructions (no_instruction 1.4-1.6 cycles per issued one).  The components are
+// read from device memory (uniform addresses, L1 hits).  Adaptive steps of 3000 and
+// 30 000 candidates through two grids and 20 modes (60 steps): 2.02 and 2.19 ms
+// inlined, 1.26 and 1.82 called.  Fixed steps of warps that are all full hide the
+// waits and lose to the call's saved registers (300 000: 15.0 and 17.7 ms); few
+// candidates per warp do not (3000: 1.83 and 1.18).  The Boris push evaluates the
+// field in a loop body and is faster inlined at every size (fixed, 300 000: 2.15
+// and 2.48 ms; adaptive 0.7 to 0.95 of the time called).
+__device__ __noinline__ f3 field_sum_call(const DevComponent *f, int n, double x, double y, double z,
+                                          const PwTab *sh) {
+    return field_sum(f, n, x, y, z, sh);
 }
 
 // A single galactic field, called without the sum's tests and loads (each some
@@ -1112,7 +1122,7 @@ __device__ __forceinline__ f3 galactic_field(const DevComponent &f, double x, do
     }
 }
 
-template <int FS, bool FUSED = false>
+template <int FS, bool FUSED = false, bool CALL = false>
 __device__ __forceinline__ f3 field_at(const DevPlan &P, double x, double y, double z,
                                        Cand *cc = nullptr, const PwTab *sh = nullptr) {
     if (FS == FS_GRID) return grid_field_t<true, false, FUSED>(P.fields[0].grid, x, y, z, cc);
@@ -1120,7 +1130,7 @@ __device__ __forceinline__ f3 field_at(const DevPlan &P, double x, double y, dou
     if (FS == FS_PLANE_WAVE) return plane_wave_field(P.fields[0].pw, x, y, z, sh);
     if (FS == FS_PLANE_WAVE_BLOCK) return plane_wave_block(P.fields[0].pw, x, y, z, P.block_warps);
     if (FS == FS_GALACTIC) return galactic_field(P.fields[0], x, y, z);
-    return field_sum(P.dev_fields, P.n_fields, x, y, z, sh);
+    return CALL ? field_sum_call(P.dev_fields, P.n_fields, x, y, z, sh) : field_sum(P.fields, P.n_fields, x, y, z, sh);
 }
 
 // Candidate::setCurrentStep (Candidate.cpp:92): the time increment s / c is
@@ -1182,12 +1192,12 @@ __device__ __forceinline__ void bp_dy(const DevPlan &P, double &x, double &y, do
     bp_rotate_drift(x, y, z, ux, uy, uz, B, kt, hh);
 }
 
-template <int FS, int MODE = 0>
+template <int FS, int MODE>
 struct BP {
     static constexpr bool kReadsStepCount = false;
     static constexpr bool kCashKarp = false;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
-    static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
+    static constexpr bool kTogether = MODE != 1;  // advance()
     struct Try {
         double step;
         int guard;
@@ -1289,7 +1299,7 @@ __constant__ double ck_eb[6] = {37. / 378. - 2825. / 27648., 0. - 0., 250. / 621
 // FP32, stage positions as FP64 base + FP32 offset, error sum in FP64.
 // Gives the end position and the direction increment, returns the direction
 // error norm.
-template <int FS>
+template <int FS, bool CALL>
 __device__ __forceinline__ double ck_try(const DevPlan &P, Cand &c, double h, float qc2E,
                                          double &xo, double &yo, double &zo, double &dux,
                                          double &duy, double &duz) {
@@ -1312,7 +1322,7 @@ __device__ __forceinline__ double ck_try(const DevPlan &P, Cand &c, double h, fl
         }
         float inv = rsqrtf(vx * vx + vy * vy + vz * vz);
         f3 vel = f3mk(vx * inv, vy * inv, vz * inv);  // unit velocity
-        f3 B = field_at<FS>(P, c.x + (double)(ox * hc), c.y + (double)(oy * hc), c.z + (double)(oz * hc), &c);
+        f3 B = field_at<FS, false, CALL>(P, c.x + (double)(ox * hc), c.y + (double)(oy * hc), c.z + (double)(oz * hc), &c);
         f3 d = cross(vel, B);
         kx[i] = vel;
         ku[i] = f3mk(d.x * qc2E, d.y * qc2E, d.z * qc2E);  // (q c / E) (c vel x B)
@@ -1328,12 +1338,12 @@ __device__ __forceinline__ double ck_try(const DevPlan &P, Cand &c, double h, fl
     return sqrt(norm2(eux, euy, euz));
 }
 
-template <int FS, int MODE = 0>
+template <int FS, int MODE, bool CALLED>
 struct CK {
     static constexpr bool kReadsStepCount = false;
     static constexpr bool kCashKarp = true;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
-    static constexpr bool kRetries = MODE != 1;  // the step controller may reject a try
+    static constexpr bool kTogether = MODE != 1 || FS == FS_GENERIC;  // advance()
     struct Try {
         double step;
         int guard;
@@ -1353,7 +1363,7 @@ struct CK {
         double step = t.step, newStep = step;
         const float qc2E = __fdividef((float)(c.q * (kCLight * kCLight)), (float)c.E);
         double xo, yo, zo, dux, duy, duz;
-        const double err = ck_try<FS>(P, c, step * kInvCLight, qc2E, xo, yo, zo, dux, duy, duz);
+        const double err = ck_try<FS, CALLED>(P, c, step * kInvCLight, qc2E, xo, yo, zo, dux, duy, duz);
         if (!on) return false;
         sc.tries++; sc.evals += 6;
         if (MODE != 1) {
@@ -1604,7 +1614,7 @@ template <int FS>
 struct SDE {
     static constexpr bool kReadsStepCount = true;  // the Philox counter
     static constexpr bool kBlockField = false;
-    static constexpr bool kRetries = false;
+    static constexpr bool kTogether = false;  // advance()
     struct Try {};
     __device__ __forceinline__ static bool begin(const DevPlan &, const DevModule &, Cand &, Try &) { return true; }
     __device__ __forceinline__ static bool attempt(const DevPlan &P, const DevModule &m, Cand &c, Try &,
@@ -1626,10 +1636,13 @@ template <class T> struct MinBlocks { static constexpr int value = 1; };
 template <int FS, int MODE> struct MinBlocks<BP<FS, MODE>> {
     static constexpr int value = MODE != 1 ? CRP_BP_ADAPTIVE_MIN_BLOCKS : FS == FS_GRID ? CRP_BP_GRID_MIN_BLOCKS : CRP_BP_FIXED_MIN_BLOCKS;
 };
-template <int FS, int MODE> struct MinBlocks<CK<FS, MODE>> { static constexpr int value = CRP_CK_MIN_BLOCKS; };
+template <int FS, int MODE, bool CALLED> struct MinBlocks<CK<FS, MODE, CALLED>> {
+    static constexpr int value = CRP_CK_MIN_BLOCKS;
+};
 template <int FS> using BPAdaptive = BP<FS, 2>;
-template <int FS> using CKFixed = CK<FS, 1>;
-template <int FS> using CKAdaptive = CK<FS, 2>;
+template <int FS> using CKFixed = CK<FS, 1, FS == FS_GENERIC>;
+template <int FS> using CKFixedInlined = CK<FS, 1, false>;  // lists of fields, warps full (step_*_ck.cu)
+template <int FS> using CKAdaptive = CK<FS, 2, FS == FS_GENERIC>;
 
 template <template <int> class Prop, int FS, int CS>
 __global__ void __launch_bounds__(128, MinBlocks<Prop<FS>>::value)

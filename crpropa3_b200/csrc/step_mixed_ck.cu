@@ -12,6 +12,11 @@ cudaError_t launch_mixed_ck_chunk(const DevPlan &P, const DevState &s, uint64_t 
     if (n == 0) return cudaSuccess;
     const DevModule &pm = P.modules[P.prop_index];
     const bool fixed = pm.min_step == pm.max_step;
+    if (fixed && fs == FS_GENERIC && lanes == 32) {  // every warp full: field_sum_call
+        mixed_chunk_kernel<CKFixedInlined, FS_GENERIC, CS_GENERIC><<<(unsigned)((n + block - 1) / block), block, 0, st>>>(
+            P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
+        return cudaGetLastError();
+    }
     return fixed ? launch_prop<CKFixed>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, lanes, st)
                  : launch_prop<CKAdaptive>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out, fs, block, lanes, st);
 }
