@@ -238,8 +238,17 @@ crp_status validate_module(const crp_module_desc &m) {
 // of its upper neighbour in z (periodic).  A trilinear gather is then four
 // aligned 256-bit loads, one sector each, where the packed cells took 24
 // scalar loads and cells padded to 16 bytes eight 128-bit ones (six sectors on
-// average).  Grids above 2^30 cells (34 GB of records) are read packed.
-constexpr size_t kPairCells = (size_t)1 << 30;
+// average).  Grids above 2^30 cells (34 GB of records) are read packed, and grids
+// whose records, from kRecordsToAsk bytes on (asking takes 0.25 ms), would take
+// more than half of the free memory: what a program allocates beside its plans
+// keeps room.  The results are the same (DevGrid::rounded).
+constexpr size_t kPairCells = (size_t)1 << 30, kRecordsToAsk = (size_t)1 << 28;
+
+bool room_for_records(size_t bytes) {
+    size_t free_bytes = 0, total = 0;
+    return bytes < kRecordsToAsk ||
+           (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && bytes <= free_bytes / 2);
+}
 
 __global__ void pair_records_kernel(const float *g, unsigned nz, unsigned cells, float4 *pairs) {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -264,8 +273,9 @@ crp_status build_grid(crp_plan *p, const crp_grid3f_desc &g, int comps, DevGrid 
     dg.pairs = nullptr;
     // records (for the trilinear gathers that read them) and values in one allocation
     void *d = nullptr;
-    const size_t records =
+    size_t records =
         comps == 3 && cells <= kPairCells && g.interpolation == CRP_INTERPOLATION_TRILINEAR ? cells * 32 : 0;
+    if (!room_for_records(records)) records = 0;
     cudaError_t e = records ? cudaMalloc(&d, records + cells * 12) : cudaErrorMemoryAllocation;
     if (e == cudaSuccess) {
         p->owned.push_back(d);

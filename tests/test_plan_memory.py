@@ -65,3 +65,23 @@ def test_same_results_where_the_pair_records_find_no_room(precision, n_extra):
     assert used < 16 * CELLS
     for name, a in want.members().items():
         np.testing.assert_array_equal(getattr(got, name), a, err_msg=name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [_abi.PRECISION_FP64, _abi.PRECISION_MIXED])
+def test_pair_records_leave_room_for_the_rest_of_the_program(precision):
+    """Free memory for a grid's values, its records and little more: the values only."""
+    import torch
+    torch.cuda.empty_cache()
+    _plan_and_bytes(_spec(precision, values=np.zeros((2, 2, 2, 3), np.float32)))  # the context's own memory
+    free = torch.cuda.mem_get_info()[0]
+    room = 12 * CELLS + 48 * CELLS
+    fill = torch.empty(free - room, dtype=torch.uint8, device="cuda")
+    try:
+        _, used = _plan_and_bytes(_spec(precision))
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert 12 * CELLS <= used < 16 * CELLS
+    _, used = _plan_and_bytes(_spec(precision))  # with the whole device free
+    assert used >= 44 * CELLS
