@@ -12,7 +12,8 @@
 //        by its odd power series;
 //   exp: t = j ln2 + u, u / 2^8 by its Taylor series, squared 8 times.
 // and rounds hi + lo once.  Valid for finite x > 0 and finite y with
-// |y log x| < 700; other inputs fall back to pow().  Host and device.
+// |y log x| < 700; other inputs fall back to pow().  Host and device, as the
+// quotients, roots and reciprocals without divisions at the end.
 #pragma once
 
 #include <cmath>
@@ -132,7 +133,7 @@ CRP_HD dd dd_exp(dd t) {
 }
 
 // x^y for normal x, |y| <= 1, to a relative error below 2^-63 and rounded, if that
-// error cannot change the rounding (true for all but 0.8 % of inputs).  The
+// error cannot change the rounding (true for all but 0.6 % of inputs).  The
 // same reductions as below, with the leading terms of each series in
 // double-double and their tails, at most 2^-12.5 of the sum, in double:
 //   log: s = (m-1)/(m+1), z = s^2 <= 0.0295: 2 s (1 + z/3 + z^2 P(z)); error of the
@@ -206,6 +207,42 @@ CRP_HD double cr_pow(double x, double y) {
     if (!(fabs(t.hi) < 700.0)) return pow(x, y);
     dd r = dd_exp(t);
     return r.hi + r.lo;
+}
+
+// a / b, rounded to nearest, for rb = 1 / b rounded to nearest (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990): the first correction leaves a quotient within one ulp, whose remainder
+// is exact, and the second rounds it correctly.  a and a / b nonzero and far
+// from the ends of the exponent range.
+CRP_HD double quotient(double a, double b, double rb) {
+    double q = a * rb;
+    q = fma(fma(-q, b, a), rb, q);
+    return fma(fma(-q, b, a), rb, q);
+}
+
+// sqrt(n2), rounded to nearest, for |n2 - 1| < 2^-27.  With n2 = 1 + e the square root
+// is 1 + e/2 - e^2/8, and e/2 is a multiple of half the spacing of doubles there:
+// the small last term only decides the ties, downwards, so rounding 1 + e/2 down
+// gives the correctly rounded root.  (On the host the directed rounding is made
+// from the exact remainder of the nearest one.)
+CRP_HD double root_near_1(double n2) {
+#ifdef __CUDA_ARCH__
+    return __fma_rd(0.5, n2, 0.5);
+#else
+    const double r = fma(0.5, n2, 0.5);
+    return fma(0.5, n2, 0.5 - r) < 0 ? nextafter(r, 0.0) : r;
+#endif
+}
+
+// 1 / r, rounded to nearest, for |r - 1| < 2^-27: 1/r = 1 - d + d^2 for r = 1 + d is
+// 2 - r with its ties rounded up.
+CRP_HD double reciprocal_near_1(double r) {
+#ifdef __CUDA_ARCH__
+    return __dsub_ru(2.0, r);
+#else
+    const double v = 2.0 - r;
+    return (2.0 - v) - r > 0 ? nextafter(v, 2.0) : v;
+#endif
 }
 
 }  // namespace crp

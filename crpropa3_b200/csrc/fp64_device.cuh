@@ -81,28 +81,16 @@ __device__ __forceinline__ double clipd(double x, double lo, double hi) { return
 // correctly rounded quotients follow from a correctly rounded reciprocal by fused
 // remainders:
 //
-// a / b, rounded to nearest, for rb = 1 / b rounded to nearest (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor",
-// 1990): the first correction leaves a quotient within one ulp, whose remainder
-// is exact, and the second rounds it correctly.  a and a / b nonzero and far
-// from the ends of the exponent range.
-__device__ __forceinline__ double quotient(double a, double b, double rb) {
-    double q = a * rb;
-    q = fma(fma(-q, b, a), rb, q);
-    return fma(fma(-q, b, a), rb, q);
-}
+// the scalar quotient, root_near_1 and reciprocal_near_1: crmath.cuh
+using crp::quotient;
 __device__ __forceinline__ d3 quotient(d3 a, double b, double rb) {
     return {quotient(a.x, b, rb), quotient(a.y, b, rb), quotient(a.z, b, rb)};
 }
 
-// u / |u| for n2 = u.u within 2^-27 of 1.  With n2 = 1 + e the square root is
-// 1 + e/2 - e^2/8, and e/2 is a multiple of half the spacing of doubles there:
-// the small last term only decides the ties, downwards, so rounding 1 + e/2 down
-// gives the correctly rounded root r.  In the same way 1/r = 1 - d + d^2 for
-// r = 1 + d is 2 - r with its ties rounded up.
+// u / |u| for n2 = u.u within 2^-27 of 1.
 __device__ __forceinline__ d3 unit_near_1(d3 u, double n2) {
-    const double r = __fma_rd(0.5, n2, 0.5);
-    return quotient(u, r, __dsub_ru(2.0, r));
+    const double r = root_near_1(n2);
+    return quotient(u, r, reciprocal_near_1(r));
 }
 
 __device__ __forceinline__ int exponent_bits(double a) { return __double2hiint(a) & 0x7fffffff; }
