@@ -1056,6 +1056,22 @@ static crp_status ensure_pipeline(crp_plan *p, uint64_t n, cudaStream_t st) {
     return CRP_OK;
 }
 
+// Candidates per warp of a chunked launch of n candidates: spread over the
+// schedulers (lanes_per_warp) but for Cash-Karp chains that lose by it.
+//   Fixed steps over one grid, mode table or galactic field: the lanes stay
+// together, and 592 partly filled warps fetch the six inlined evaluations' code on
+// every SM (3000 candidates x 60 steps over 64^3 cells, full warps and spread: mixed,
+// clipped grid 0.234 and 0.266 ms; FP64, periodic grid 0.232 and 0.259).
+//   Tricubic grids above 8 per warp: 64 cells per gather and the code of six of them
+// (adaptive, mixed: 8000 candidates 4.83 and 7.59 ms, 3000 4.83 and 4.20).
+static int launch_lanes(const crp_plan *p, uint64_t n) {
+    const int lanes = lanes_per_warp(n, p->num_sms, kSpreadWarpsPerSm);
+    const DevModule &m = p->dev.modules[p->dev.prop_index];
+    if (m.propagator != CRP_PROP_CK) return lanes;
+    if (p->fs == FS_GRID && p->dev.fields[0].grid.interp == CRP_INTERPOLATION_TRICUBIC) return lanes <= 8 ? lanes : 32;
+    return m.min_step == m.max_step && p->fs != FS_GENERIC ? 32 : lanes;
+}
+
 // What crp_run() asks of run_device(): the arrays are the plan's own, the input
 // chunks (or null), and where the results go (or null): a copy of `bytes` queued
 // behind the first launch, so that a run of one launch waits once; `copied`:
@@ -1133,7 +1149,7 @@ static crp_status run_device(crp_plan *p, const crp_candidates *c, uint64_t n, c
             if (ls) return ls;
             launches++;  // the key kernel (the radix sort is CUB's)
         }
-        const int lanes = lanes_per_warp(n_threads, p->num_sms, kSpreadWarpsPerSm);
+        const int lanes = launch_lanes(p, n_threads);
         auto step = [&](uint64_t nt, const uint32_t *li, cudaStream_t ss) {
             return (p->precision == CRP_PRECISION_FP64)
                 ? launch_fp64_chunk(p->dev, s, nt, spl, o.max_steps, p->d_cnt, rec, li, list_out, p->fs, block, lanes, ss)
