@@ -47,7 +47,7 @@ struct AdjGrid {
     const float *g;
     int nx, ny, nz;
     bool pow2;  // every dimension a power of two: indices wrap with a mask
-    double gox, goy, goz, sx, sy, sz;
+    double gox, goy, goz;
     double isx, isy, isz;  // 1 / spacing
 };
 
@@ -446,8 +446,7 @@ AdjGrid make_grid(const crp_adjoint_desc *d) {
     G.gox = d->origin[0] + d->spacing[0] / 2;
     G.goy = d->origin[1] + d->spacing[1] / 2;
     G.goz = d->origin[2] + d->spacing[2] / 2;
-    G.sx = d->spacing[0]; G.sy = d->spacing[1]; G.sz = d->spacing[2];
-    G.isx = 1.0 / G.sx; G.isy = 1.0 / G.sy; G.isz = 1.0 / G.sz;
+    G.isx = 1.0 / d->spacing[0]; G.isy = 1.0 / d->spacing[1]; G.isz = 1.0 / d->spacing[2];
     return G;
 }
 

@@ -52,8 +52,9 @@ inline int lanes_per_warp(uint64_t n, int num_sms, int warps_per_sm) {
     return l < 1 ? 1 : l > 32 ? 32 : (int)l;
 }
 
-// Runs up to this size ask for the next grid cell ahead (step_*_bp.cu).
-constexpr uint64_t kAskAheadCandidates = 592 * 40;
+// Runs up to 40 candidates per scheduler ask for the next grid cell ahead
+// (step_*_bp.cu).
+inline bool ask_ahead(uint64_t n, int num_sms) { return n <= 160 * (uint64_t)num_sms; }
 
 // Chunked launches over a PlaneWaveTurbulence field summed by the block
 // (FS_PLANE_WAVE_BLOCK).  The largest table taken: 98 KB in the FP64 form, two blocks

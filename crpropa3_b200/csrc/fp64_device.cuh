@@ -539,6 +539,7 @@ __device__ __forceinline__ void set_direction(Cand &c, d3 uo) {
 
 template <int FS, int MODE>
 struct BP {
+    static constexpr bool kBorisKernel = MODE == 1;  // its own kernel for CS_PM over FS_GRID_PERIODIC
     static constexpr bool kReadsStepCount = false;
     static constexpr bool kCashKarp = false;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
@@ -667,6 +668,7 @@ __device__ __forceinline__ void ck_try(const DevPlan &P, d3 x, d3 u, double h, d
 
 template <int FS, int MODE, bool CALLED>
 struct CK {
+    static constexpr bool kBorisKernel = false;  // its own kernel for CS_PM over FS_GRID_PERIODIC
     static constexpr bool kReadsStepCount = false;
     static constexpr bool kCashKarp = true;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
@@ -755,6 +757,7 @@ __device__ __forceinline__ void sde_try(const DevPlan &P, d3 PosIn, d3 &POut, d3
 
 template <int FS>
 struct SDE {
+    static constexpr bool kBorisKernel = false;  // its own kernel for CS_PM over FS_GRID_PERIODIC
     static constexpr bool kReadsStepCount = true;  // the Philox counter
     static constexpr bool kBlockField = false;
     static constexpr bool kTogether = false;  // advance()
@@ -968,8 +971,11 @@ cudaError_t launch_prop(const DevPlan &P, const DevState &s, uint64_t n, int max
     const uint64_t slots = (uint64_t)(block / 32) * (uint64_t)lanes;
     const unsigned grid = (unsigned)((n + slots - 1) / slots);
     for_signature(fs, P.shape, [&](auto f, auto c) {
-        fp64_chunk_kernel<Prop, decltype(f)::value, decltype(c)::value><<<grid, block, 0, st>>>(
-            P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
+        constexpr int FS = decltype(f)::value, CS = decltype(c)::value;
+        // (fp64_boris_kernel takes these)
+        if constexpr (!(Prop<FS>::kBorisKernel && FS == FS_GRID_PERIODIC && CS == CS_PM))
+            fp64_chunk_kernel<Prop, FS, CS><<<grid, block, 0, st>>>(P, s, n, lanes, max_steps, step_cap, cnt, rec, perm,
+                                                                     perm_out);
     });
     return cudaGetLastError();
 }

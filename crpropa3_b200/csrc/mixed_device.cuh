@@ -77,14 +77,11 @@ __device__ __forceinline__ int wrap(int i, int n, bool pow2) {
 
 // Trilinear Grid3f interpolation: FP64 cell coordinates, FP32 weights and
 // values (the reference's own interpolation arithmetic is FP32, Grid.h:571).
-// With a cell cache (FS_GRID kernels) the 8 corners are loaded only when the
-// cell changes.
-// PER: the grid is periodic with power-of-two dimensions, has no clipVolume
-// and has pair records (FS_GRID_PERIODIC): those branches are compiled out.
-// The periodic power-of-two case in two parts: grid_cell_load finds the
-// cell of (x, y, z) and, when it is not the cached one, loads its 8 corners
-// into the candidate's cache; grid_cell_interp forms the trilinear sum from
-// the cache.
+//
+// Periodic power-of-two grids without clipVolume and with pair records
+// (FS_GRID_PERIODIC) in two parts: grid_cell_load finds the cell of (x, y, z) and,
+// when it is not the cached one, loads its 8 corners into the candidate's cache;
+// grid_cell_interp forms the trilinear sum from the cache.
 struct CellFrac { float fx0, fy0, fz0; };
 
 template <bool AHEAD = false>
@@ -123,22 +120,21 @@ __device__ __forceinline__ f3 grid_cell_interp(const CellFrac &f, const float (&
     return f3mk(bx, by, bz);
 }
 
+// Any grid.  CACHE (FS_GRID kernels): the 8 corners are loaded only when the cell
+// changes.
 // FUSED: the cell fraction from the unrounded product of position and inverse
 // spacing (one multiply-add), as the fixed-step Boris kernels over any grid
 // form it; otherwise, and for grids marked `rounded` (FS_GRID_PERIODIC's, where
-// their pair records found no room), from the rounded coordinate.  Written out so that it does
-// not depend on how the compiler contracts the expression in each kernel.
-template <bool CACHE, bool PER = false, bool FUSED = false>
+// their pair records found no room), from the rounded coordinate.  Written out so
+// that it does not depend on how the compiler contracts the expression in each
+// kernel.
+template <bool CACHE, bool FUSED = false>
 __device__ __forceinline__ f3 grid_field_t(const DevGrid &g, double x, double y, double z, Cand *cc) {
-    if (CACHE && PER) {
-        const CellFrac f = grid_cell_load(g, x, y, z, cc->tag, cc->corner);
-        return grid_cell_interp(f, cc->corner);
-    }
-    if (!PER && g.interp != CRP_INTERPOLATION_TRILINEAR) {  // tricubic, nearest (Grid.h:328-331)
+    if (g.interp != CRP_INTERPOLATION_TRILINEAR) {  // tricubic, nearest (Grid.h:328-331)
         const gi3 v = gi_vector_other(g, x, y, z);
         return f3mk(v.x, v.y, v.z);
     }
-    if (!PER && g.clip_volume) {
+    if (g.clip_volume) {
         bool in = (x >= g.ox) && (x <= g.ex) && (y >= g.oy) && (y <= g.ey) && (z >= g.oz) && (z <= g.ez);
         if (!in) return f3mk(0.f, 0.f, 0.f);
     }
@@ -155,7 +151,7 @@ __device__ __forceinline__ f3 grid_field_t(const DevGrid &g, double x, double y,
         fz0 = (float)__dsub_rn(rz, flz);
     }
     int ix0, ix1, iy0, iy1, iz0, iz1;
-    if (!PER && g.reflective) {
+    if (g.reflective) {
         double r[3] = {rx, ry, rz};
         int n[3] = {g.nx, g.ny, g.nz}, lo[3], hi[3];
         float f[3];
@@ -176,27 +172,25 @@ __device__ __forceinline__ f3 grid_field_t(const DevGrid &g, double x, double y,
         ix0 = lo[0]; ix1 = hi[0]; iy0 = lo[1]; iy1 = hi[1]; iz0 = lo[2]; iz1 = hi[2];
         fx0 = f[0]; fy0 = f[1]; fz0 = f[2];
     } else {
-        bool p2 = PER || g.pow2 != 0;
+        const bool p2 = g.pow2 != 0;
         ix0 = wrap((int)flx, g.nx, p2); ix1 = (ix0 + 1 == g.nx) ? 0 : ix0 + 1;
         iy0 = wrap((int)fly, g.ny, p2); iy1 = (iy0 + 1 == g.ny) ? 0 : iy0 + 1;
         iz0 = wrap((int)flz, g.nz, p2); iz1 = (iz0 + 1 == g.nz) ? 0 : iz0 + 1;
     }
     const float fx1 = 1.f - fx0, fy1 = 1.f - fy0, fz1 = 1.f - fz0;
-    // cell indices: 32-bit for FS_GRID_PERIODIC grids (fewer than 2^31 cells)
-    using Index = typename std::conditional<PER, unsigned, size_t>::type;
-    const Index sy = (Index)g.nz, sx = (Index)g.ny * (Index)g.nz;
-    const Index b00 = (Index)ix0 * sx + (Index)iy0 * sy, b10 = (Index)ix1 * sx + (Index)iy0 * sy;
-    const Index b01 = (Index)ix0 * sx + (Index)iy1 * sy, b11 = (Index)ix1 * sx + (Index)iy1 * sy;
-    const Index idx[8] = {b00 + iz0, b10 + iz0, b01 + iz0, b00 + iz1, b10 + iz1, b01 + iz1, b11 + iz0, b11 + iz1};
+    const size_t sy = (size_t)g.nz, sx = (size_t)g.ny * (size_t)g.nz;
+    const size_t b00 = (size_t)ix0 * sx + (size_t)iy0 * sy, b10 = (size_t)ix1 * sx + (size_t)iy0 * sy;
+    const size_t b01 = (size_t)ix0 * sx + (size_t)iy1 * sy, b11 = (size_t)ix1 * sx + (size_t)iy1 * sy;
+    const size_t idx[8] = {b00 + iz0, b10 + iz0, b01 + iz0, b00 + iz1, b10 + iz1, b01 + iz1, b11 + iz0, b11 + iz1};
     const float w[8] = {fx1 * fy1 * fz1, fx0 * fy1 * fz1, fx1 * fy0 * fz1, fx1 * fy1 * fz0,
                         fx0 * fy1 * fz0, fx1 * fy0 * fz0, fx0 * fy0 * fz1, fx0 * fy0 * fz0};
     float lc[8][3];
     float (*c)[3] = CACHE ? cc->corner : lc;
     const long long k0 = (long long)idx[0], k7 = (long long)idx[7];
     if (!CACHE || k0 != cc->cell0 || k7 != cc->cell7) {
-        if (PER || g.pairs) {
+        if (g.pairs) {
             load_corner_pairs<CACHE>(g.pairs, b00, b10, b01, b11, iz0, c);
-            if (!PER && iz1 == iz0) {  // the reflective edge: no upper neighbour
+            if (iz1 == iz0) {  // the reflective edge: no upper neighbour
 #pragma unroll
                 for (int a = 0; a < 3; a++) { c[3][a] = c[0][a]; c[4][a] = c[1][a]; c[5][a] = c[2][a]; c[7][a] = c[6][a]; }
             }
@@ -1125,8 +1119,11 @@ __device__ __forceinline__ f3 galactic_field(const DevComponent &f, double x, do
 template <int FS, bool FUSED = false, bool CALL = false>
 __device__ __forceinline__ f3 field_at(const DevPlan &P, double x, double y, double z,
                                        Cand *cc = nullptr, const PwTab *sh = nullptr) {
-    if (FS == FS_GRID) return grid_field_t<true, false, FUSED>(P.fields[0].grid, x, y, z, cc);
-    if (FS == FS_GRID_PERIODIC) return grid_field_t<true, true>(P.fields[0].grid, x, y, z, cc);
+    if (FS == FS_GRID) return grid_field_t<true, FUSED>(P.fields[0].grid, x, y, z, cc);
+    if (FS == FS_GRID_PERIODIC) {
+        const CellFrac f = grid_cell_load(P.fields[0].grid, x, y, z, cc->tag, cc->corner);
+        return grid_cell_interp(f, cc->corner);
+    }
     if (FS == FS_PLANE_WAVE) return plane_wave_field(P.fields[0].pw, x, y, z, sh);
     if (FS == FS_PLANE_WAVE_BLOCK) return plane_wave_block(P.fields[0].pw, x, y, z, P.block_warps);
     if (FS == FS_GALACTIC) return galactic_field(P.fields[0], x, y, z);
@@ -1194,6 +1191,7 @@ __device__ __forceinline__ void bp_dy(const DevPlan &P, double &x, double &y, do
 
 template <int FS, int MODE>
 struct BP {
+    static constexpr bool kBorisKernel = MODE == 1;  // its own kernel for CS_PM over FS_GRID_PERIODIC
     static constexpr bool kReadsStepCount = false;
     static constexpr bool kCashKarp = false;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
@@ -1340,6 +1338,7 @@ __device__ __forceinline__ double ck_try(const DevPlan &P, Cand &c, double h, fl
 
 template <int FS, int MODE, bool CALLED>
 struct CK {
+    static constexpr bool kBorisKernel = false;  // its own kernel for CS_PM over FS_GRID_PERIODIC
     static constexpr bool kReadsStepCount = false;
     static constexpr bool kCashKarp = true;
     static constexpr bool kBlockField = true;  // takes its field from the block (attempt's `on`)
@@ -1612,6 +1611,7 @@ __device__ __forceinline__ bool sde_co_consume(const DevPlan &P, const DevModule
 // run to completion, field evaluations in place.
 template <int FS>
 struct SDE {
+    static constexpr bool kBorisKernel = false;  // its own kernel for CS_PM over FS_GRID_PERIODIC
     static constexpr bool kReadsStepCount = true;  // the Philox counter
     static constexpr bool kBlockField = false;
     static constexpr bool kTogether = false;  // advance()
@@ -1750,8 +1750,11 @@ cudaError_t launch_prop(const DevPlan &P, const DevState &s, uint64_t n, int max
     const uint64_t slots = (uint64_t)(block / 32) * (uint64_t)lanes;
     const unsigned grid = (unsigned)((n + slots - 1) / slots);
     for_signature(fs, P.shape, [&](auto f, auto c) {
-        mixed_chunk_kernel<Prop, decltype(f)::value, decltype(c)::value><<<grid, block, 0, st>>>(
-            P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
+        constexpr int FS = decltype(f)::value, CS = decltype(c)::value;
+        // (mixed_boris_kernel takes these)
+        if constexpr (!(Prop<FS>::kBorisKernel && FS == FS_GRID_PERIODIC && CS == CS_PM))
+            mixed_chunk_kernel<Prop, FS, CS><<<grid, block, 0, st>>>(P, s, n, lanes, max_steps, step_cap, cnt, rec, perm,
+                                                                     perm_out);
     });
     return cudaGetLastError();
 }

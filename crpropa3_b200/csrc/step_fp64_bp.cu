@@ -16,9 +16,9 @@ cudaError_t launch_fp64_bp_chunk(const DevPlan &P, const DevState &s, uint64_t n
         const uint64_t slots = (uint64_t)(block / 32) * (uint64_t)lanes;
         const unsigned grid = (unsigned)((n + slots - 1) / slots);
         // about one warp per scheduler or less (40 candidates for each): nothing else
-        // hides the gathers' latency (256^3 grid, 1000 steps, mixed: 2000 candidates
-        // 0.81 -> 0.68 ms, 20 011 0.79 -> 0.76 ms; 50 000 lose, 1.02 -> 1.19 ms)
-        if (n <= kAskAheadCandidates)
+        // hides the gathers' latency (256^3 grid, 1000 steps: 2000 candidates 0.89 -> 0.82 ms,
+        // 20 011 1.14 -> 1.10 ms; 50 000 lose, 1.26 -> 1.32 ms)
+        if (ask_ahead(n, P.num_sms))
             fp64_boris_kernel<BorisPush<true>><<<grid, block, 0, st>>>(
                 P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
         else

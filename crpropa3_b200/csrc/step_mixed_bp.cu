@@ -18,7 +18,7 @@ cudaError_t launch_mixed_bp_chunk(const DevPlan &P, const DevState &s, uint64_t 
         // about one warp per scheduler or less (40 candidates for each): nothing else
         // hides the gathers' latency (256^3 grid, 1000 steps, mixed: 2000 candidates
         // 0.81 -> 0.68 ms, 20 011 0.79 -> 0.76 ms; 50 000 lose, 1.02 -> 1.19 ms)
-        if (n <= kAskAheadCandidates)
+        if (ask_ahead(n, P.num_sms))
             mixed_boris_kernel<BorisPush<true>><<<grid, block, 0, st>>>(
                 P, s, n, lanes, max_steps, step_cap, cnt, rec, perm, perm_out);
         else
