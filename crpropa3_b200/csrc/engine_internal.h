@@ -57,9 +57,10 @@ inline int lanes_per_warp(uint64_t n, int num_sms, int warps_per_sm) {
 inline bool ask_ahead(uint64_t n, int num_sms) { return n <= 160 * (uint64_t)num_sms; }
 
 // Chunked launches over a PlaneWaveTurbulence field summed by the block
-// (FS_PLANE_WAVE_BLOCK).  The largest table taken: 98 KB in the FP64 form, two blocks
-// per SM beside the kernel's own 11 KB.
-constexpr int kWaveMaxModes = 1365;
+// (FS_PLANE_WAVE_BLOCK).  The largest tables taken are the ones of which two blocks
+// fit on an SM beside the kernel's own arrays: 98 KB (FP64, 11 KB beside it) and
+// 102 KB (mixed, 9 KB).
+constexpr int kWaveMaxModesFp64 = 1365, kWaveMaxModesMixed = 2600;
 // Blocks per SM that the kernels' registers are held to.  FP64 Cash-Karp spills 300 B
 // at 4 (14 000 candidates x 200 modes: 1.45 ms, 1.23 at 3); the FP64 push loses at 3.
 // The mixed adaptive push is faster at 3 below 37 888 candidates (3000 x 200 modes:
@@ -94,7 +95,7 @@ inline uint64_t wave_blocks_per_sm(int n_modes, bool fp64, bool ck) {
 // the faster up to 500 modes (37 800 x 100 modes: 0.25 ms, 0.29 at 32, 0.32 at 64; x
 // 500: 1.06 and 0.98; with an observer 37 000 x 40 modes: 1.04 and 0.80 at 64).
 inline int wave_block_warps(uint64_t n, int n_modes, int num_sms, bool fp64, bool ck, bool pm) {
-    if (n_modes < (fp64 ? 32 : 8) || n_modes > kWaveMaxModes) return 0;
+    if (n_modes < (fp64 ? 32 : 8) || n_modes > (fp64 ? kWaveMaxModesFp64 : kWaveMaxModesMixed)) return 0;
     const uint64_t sms = (uint64_t)num_sms, per_sm = wave_blocks_per_sm(n_modes, fp64, ck);
     auto blocks = [n](int warps) { return (n + 32 * (uint64_t)warps - 1) / (32 * (uint64_t)warps); };
     if (blocks(1) <= per_sm * sms) return 1;

@@ -1725,7 +1725,7 @@ cudaError_t launch_waves(DevPlan P, const DevState &s, uint64_t n, int max_steps
     const unsigned grid = (unsigned)((n + 32 * warps - 1) / (32 * warps));
     auto launch = [&](auto c) {
         auto kernel = mixed_wave_kernel<Prop, decltype(c)::value>;
-        const cudaError_t e = allow_shared<(size_t)((kWaveMaxModes + 1) / 2) * 80>(kernel);
+        const cudaError_t e = allow_shared<(size_t)((kWaveMaxModesMixed + 1) / 2) * 80>(kernel);
         if (e != cudaSuccess) return e;
         kernel<<<grid, kBatchThreads, smem, st>>>(P, s, n, max_steps, step_cap, cnt, rec, perm, perm_out);
         return cudaGetLastError();

@@ -16,7 +16,7 @@ int main() {
     for (int sms : {1, 148, 160})
         for (int fp64 = 0; fp64 < 2; fp64++)
             for (int ck = 0; ck < 2; ck++)
-                for (int m = 1; m <= 1400; m += m < 70 ? 1 : 7)
+                for (int m = 1; m <= 2700; m += m < 70 ? 1 : 7)
                     for (uint64_t n = 1; n < 400000; n += 1 + n / 23) {
                         const int w = crp::wave_block_warps(n, m, sms, fp64, ck, n % 2);
                         const uint64_t blocks = w ? (n + 32 * w - 1) / (32 * w) : 0;
@@ -49,8 +49,9 @@ NAMES = ("x", "y", "z", "dx", "dy", "dz", "px", "py", "pz", "trajectory_length",
 BLOCKS = [(_abi.PRECISION_FP64, 129, 32), (_abi.PRECISION_FP64, 18945, 101), (_abi.PRECISION_FP64, 65, 1365),
           (_abi.PRECISION_FP64, 9473, 1365), (_abi.PRECISION_MIXED, 129, 8), (_abi.PRECISION_MIXED, 65, 1365),
           (_abi.PRECISION_MIXED, 18945, 200), (_abi.PRECISION_MIXED, 37889, 33),
+          (_abi.PRECISION_MIXED, 65, 2600),
           # thread by thread: one mode more than the largest table, and one fewer than the least
-          (_abi.PRECISION_FP64, 65, 1366), (_abi.PRECISION_MIXED, 65, 1366), (_abi.PRECISION_FP64, 65, 31)]
+          (_abi.PRECISION_FP64, 65, 1366), (_abi.PRECISION_MIXED, 65, 2601), (_abi.PRECISION_FP64, 65, 31)]
 
 
 @pytest.mark.gpu
