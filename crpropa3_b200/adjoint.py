@@ -4,10 +4,10 @@
 for candidates with initial momenta p0 (n, 3) [kg m/s] propagated with a
 fixed-step Boris push through a periodic Grid3f whose values `grid`
 (nx, ny, nz, 3) float32 are differentiated too.  The forward pass calls
-crp_bp_forward_loss (no checkpoints kept); backward calls crp_bp_adjoint,
-which recomputes the forward pass with FP64 checkpoints every
-`checkpoint_every` steps and runs the hand-written adjoint.  PyTorch is only
-the autograd wrapper: both passes are the engine's CUDA kernels.
+crp_bp_adjoint_forward, which keeps FP64 checkpoints every
+`checkpoint_every` steps; backward calls crp_bp_adjoint_backward, the
+hand-written adjoint, which recomputes the steps between them.  PyTorch is
+only the autograd wrapper: both passes are the engine's CUDA kernels.
 
 With p0 = (E/c) u0:  dL/dp0 = (I - u0 u0^T) dL/du0 / |p0| + c u0 dL/dE.
 """

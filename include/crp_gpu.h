@@ -507,7 +507,9 @@ enum crp_run_mode {
 
 typedef struct crp_run_opts {
     int32_t mode;
-    int32_t block_size;        /* 0: autotuned; else a multiple of 32 up to 128 */
+    int32_t block_size;        /* 0: autotuned; else a multiple of 32 up to 128.  Chunked runs that
+                                  sum PlaneWaveTurbulence modes by the block take 128 whatever it
+                                  says (the results do not depend on it) */
     int32_t ctas_per_sm;       /* 0: autotuned (persistent mode) */
     int32_t steps_per_launch;  /* 0: default (chunked mode) */
     int32_t refill_threshold;  /* persistent: lanes idle before a warp refills, 0: autotuned */
@@ -539,7 +541,10 @@ crp_status crp_device_count(int32_t *count);
 /* Plan: validates the chain the way the reference constructors and setters
  * do (PropagationCK.cpp:163-190, PropagationBP.cpp:148-178,
  * DiffusionSDE.cpp:280-320), uploads grids and wave-mode tables to the
- * current device. */
+ * current device.  A Grid3f takes 12 bytes of device memory per cell.  A trilinear
+ * one of up to 2^30 cells takes 32 more for the records its gathers read, from
+ * 256 MB on only where they are at most half of the free memory; the results do
+ * not depend on it. */
 crp_status crp_plan_create(const crp_plan_desc *desc, crp_plan **plan);
 crp_status crp_plan_destroy(crp_plan *plan);
 
@@ -547,8 +552,10 @@ crp_status crp_plan_destroy(crp_plan *plan);
  * arrays: copied to the device and back inside the call; in the chunked mode,
  * from 2^18 candidates on, the inputs go in 8 chunks on a copy stream and the
  * first launch starts on each chunk as it arrives (the first launch's
- * device_ms then includes that wait).  Pinned host arrays give the fastest
- * copies. */
+ * device_ms then includes that wait).  Up to 2^15 candidates, pageable arrays
+ * are gathered in a pinned buffer that the plan keeps (145 bytes per candidate),
+ * one copy each way.  Other arrays are copied one by one in the order of the
+ * run's stream; above that size pinned ones give the fastest copies. */
 crp_status crp_run(crp_plan *plan, const crp_candidates *host, uint64_t n,
                    const crp_run_opts *opts, crp_run_stats *stats);
 /* Same, on device-resident arrays, asynchronous with respect to the host
@@ -617,7 +624,8 @@ typedef struct crp_adjoint_io {
     double *grad_grid;             /* out: dL/d(grid value), nx*ny*nz*3, may be NULL */
 } crp_adjoint_io;
 
-/* Bytes of device workspace crp_bp_adjoint needs for n candidates. */
+/* Bytes of device workspace crp_bp_adjoint needs for n candidates: 48 per
+ * candidate and checkpoint, 24 per cell, and under 1 KB. */
 crp_status crp_bp_adjoint_workspace(const crp_adjoint_desc *desc, uint64_t n, size_t *bytes);
 /* Forward pass only: loss (and final directions). */
 crp_status crp_bp_forward_loss(const crp_adjoint_desc *desc, const crp_adjoint_io *io, void *stream);
