@@ -1298,14 +1298,15 @@ crp_status crp_run(crp_plan *p, const crp_candidates *h, uint64_t n, const crp_r
         cudaPointerAttributes a{};
         staged = cudaPointerGetAttributes(&a, members[k].host) == cudaSuccess && a.type == cudaMemoryTypeUnregistered;
     }
+    if (staged && p->staging_bytes < off) {
+        if (p->staging) { cudaFreeHost(p->staging); p->staging = nullptr; p->staging_bytes = 0; }
+        staged = cudaMallocHost(&p->staging, off) == cudaSuccess;  // no pinned memory left: copied one by one
+        if (staged) p->staging_bytes = off;
+        else p->staging = nullptr;
+    }
     cudaGetLastError();
     HostRun host{pipe ? &chunks : nullptr, nullptr, nullptr, 0, false};
     if (staged) {
-        if (p->staging_bytes < off) {
-            if (p->staging) { cudaFreeHost(p->staging); p->staging = nullptr; p->staging_bytes = 0; }
-            CUDA_TRY(cudaMallocHost(&p->staging, off));
-            p->staging_bytes = off;
-        }
         for (int k = 0; k < n_members; k++)
             memcpy(p->staging + (static_cast<char *>(members[k].dev) - base), members[k].host, members[k].size * n);
         CUDA_TRY(cudaMemcpyAsync(base, p->staging, off, cudaMemcpyHostToDevice, st));
