@@ -1189,7 +1189,8 @@ __device__ __forceinline__ void bp_dy(const DevPlan &P, double &x, double &y, do
     bp_rotate_drift(x, y, z, ux, uy, uz, B, kt, hh);
 }
 
-template <int FS, int MODE>
+// FUSED: grid_field_t, for fixed steps.
+template <int FS, int MODE, bool FUSED>
 struct BP {
     static constexpr bool kBorisKernel = MODE == 1;  // its own kernel for CS_PM over FS_GRID_PERIODIC
     static constexpr bool kReadsStepCount = false;
@@ -1219,7 +1220,7 @@ struct BP {
         const float kq = boris_kq(c.q, c.E);
         double xo = c.x, yo = c.y, zo = c.z, uxo = c.dx, uyo = c.dy, uzo = c.dz;
         if (MODE == 1) {
-            bp_dy<FS, true>(P, xo, yo, zo, uxo, uyo, uzo, step, kq * (float)step, &c);
+            bp_dy<FS, FUSED>(P, xo, yo, zo, uxo, uyo, uzo, step, kq * (float)step, &c);
             if (!on) return false;
             sc.tries++; sc.evals++;
         } else {
@@ -1629,17 +1630,20 @@ struct SDE {
 
 // step-mode variants selected by the launcher from min_step == max_step, so
 // that a fixed-step kernel carries no adaptive-controller registers
-template <int FS> using BPFixed = BP<FS, 1>;
+// (the persistent kernels form their cell fractions from rounded coordinates over
+// any grid, as the adaptive ones do)
+template <int FS> using BPFixed = BP<FS, 1, true>;
+template <int FS> using BPFixedPersistent = BP<FS, 1, false>;
 // resident blocks of 128 threads per SM the register budget is sized for:
 // the fixed-step Boris push is latency bound on its gathers and wants warps
 template <class T> struct MinBlocks { static constexpr int value = 1; };
-template <int FS, int MODE> struct MinBlocks<BP<FS, MODE>> {
+template <int FS, int MODE, bool FUSED> struct MinBlocks<BP<FS, MODE, FUSED>> {
     static constexpr int value = MODE != 1 ? CRP_BP_ADAPTIVE_MIN_BLOCKS : FS == FS_GRID ? CRP_BP_GRID_MIN_BLOCKS : CRP_BP_FIXED_MIN_BLOCKS;
 };
 template <int FS, int MODE, bool CALLED> struct MinBlocks<CK<FS, MODE, CALLED>> {
     static constexpr int value = CRP_CK_MIN_BLOCKS;
 };
-template <int FS> using BPAdaptive = BP<FS, 2>;
+template <int FS> using BPAdaptive = BP<FS, 2, false>;
 template <int FS> using CKFixed = CK<FS, 1, FS == FS_GENERIC>;
 template <int FS> using CKFixedInlined = CK<FS, 1, false>;  // lists of fields, warps full (step_*_ck.cu)
 template <int FS> using CKAdaptive = CK<FS, 2, FS == FS_GENERIC>;

@@ -34,7 +34,7 @@ cudaError_t launch_mixed_bp_persistent(const DevPlan &P, const DevState &s, cons
                                        DevCounters *cnt, const DevRecords &rec, int fs, int grid, cudaStream_t st) {
     const DevModule &pm = P.modules[P.prop_index];
     const bool fixed = pm.min_step == pm.max_step;
-    return fixed ? launch_persistent_prop<BPFixed>(P, s, a, cnt, rec, fs, grid, st)
+    return fixed ? launch_persistent_prop<BPFixedPersistent>(P, s, a, cnt, rec, fs, grid, st)
                  : launch_persistent_prop<BPAdaptive>(P, s, a, cnt, rec, fs, grid, st);
 }
 

@@ -37,3 +37,28 @@ def test_saturated_cell_indices(precision, prop):
         got.append(dev.to_host())
     for name in NAMES:
         np.testing.assert_array_equal(getattr(got[0], name), getattr(got[1], name), err_msg=name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("far", [1e6, 1e12])
+def test_persistent_fixed_push_rounds_its_coordinates(far):
+    """Persistent launches of the mixed fixed push over a general grid: the cell fractions of
+    the periodic power-of-two grid, far from the origin too, and no NaN at 10^300 m."""
+    from crpropa3_b200.engine import Plan
+    grid = random_grid(np.random.default_rng(8), 16, 3e-13)
+    rng = np.random.default_rng(10)
+    c = protons(rng, 500, emin=0.1 * U.EeV)
+    c.set_position(rng.uniform(-far, far, (500, 3)) * 10 * U.kpc)
+    got = []
+    for values in (grid, np.tile(grid, (3, 3, 3, 1))):
+        plan = Plan(P.ChainSpec([P.GridField(values, (0, 0, 0), (10 * U.kpc,) * 3)],
+                                [P.Propagation(_abi.PROP_BP, 0.42, 1 * U.kpc, 1 * U.kpc), P.MaxTrajectoryLength(60 * U.kpc)],
+                                precision=_abi.PRECISION_MIXED))
+        dev = c.to_device()
+        plan.run(dev, mode=_abi.MODE_PERSISTENT)
+        got.append(dev.to_host())
+    for name in NAMES:
+        np.testing.assert_array_equal(getattr(got[0], name), getattr(got[1], name), err_msg=name)
+    c.x[::3] = 1e300
+    plan.run(c, mode=_abi.MODE_PERSISTENT)
+    assert np.isfinite(c.position()).all()
